@@ -8,7 +8,16 @@
  * applied to every query row, with the probabilities rounded to bf16 before
  * they multiply V, as every tensor-core flash attention does.  O is rescaled
  * only when a row's maximum has grown by more than 2^8 since the value in use;
- * the final division by the row sum makes the result independent of it.
+ * the final division by the row sum makes the result independent of it, but for
+ * where the probabilities round.
+ *
+ * Sequences of whole pairs of Q tiles start from a maximum of zero.  Those of an
+ * odd number of tiles (kBy64) round as 64-key tiles do: their maximum starts as
+ * that of a row's first 64 keys, and the row sums are kept in the same order.  The
+ * two choices are equally far from 64 bits (2.33e-3 of bf16 rounding) and 3.2e-3
+ * from each other; a sequence keeps the one its results have always had.
+ * [2, 32, 1152, 128] without a mask takes 69.3 us that way and 67.6 from a maximum
+ * of zero; kernels of 64-key tiles took 88.2.
  *
  * A CTA owns two tiles of 128 query rows of one (batch, head), or the one that an
  * odd number of tiles leaves over, and walks KV tiles of 128 rows:
@@ -167,11 +176,98 @@ probabilities_stored(uint32_t s_tmem, float scale_log2, float neg_m) {
   return (part4[0] + part4[1]) + (part4[2] + part4[3]);
 }
 
-/* The largest of a row's 128 scores (as stored, before scaling). */
-__device__ __forceinline__ float row_max(uint32_t s_tmem) {
+/* The row sums of 32 columns' probabilities in the order of 64-key tiles: each half of
+   such a tile has a sum of its own. `a`, `b`: exponentials of columns e .. e + 3. */
+struct HalfSums {
+  float l[2] = {0.0f, 0.0f};
+  uint64_t part[2]; /* four chains, two to a word */
+  __device__ __forceinline__ void begin() { part[0] = part[1] = 0; }
+  __device__ __forceinline__ void add(int e, float a0, float a1, float b0, float b1) {
+    part[(e >> 2) & 1] = add2(part[(e >> 2) & 1], add2(pair_of(a0, b0), pair_of(a1, b1)));
+  }
+  /* 32 columns are done, of half c & 1; fix: what the sum so far is scaled by */
+  __device__ __forceinline__ void end(int c, float fix) {
+    float p0, p1, p2, p3;
+    halves_of(part[0], p0, p1);
+    halves_of(part[1], p2, p3);
+    l[c & 1] = fmaf(l[c & 1], fix, (p0 + p1) + (p2 + p3));
+  }
+};
+
+/* probabilities() with those sums. */
+__device__ __forceinline__ void
+probabilities_by64(uint32_t s_tmem, float scale_log2, float neg_m,
+                   uint32_t (&packed)[BKV / 2], float &rel_max, HalfSums &sums) {
+  uint32_t raw[2][32];
+  float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  const uint64_t scale2 = pair_of(scale_log2, scale_log2);
+  const uint64_t negm2 = pair_of(neg_m, neg_m);
+  ptx::tmem_ld_32x32b_x32(s_tmem, raw[0]);
+#pragma unroll
+  for (int c = 0; c < BKV / 32; ++c) {
+    ptx::tmem_ld_wait_for(raw[c & 1]);
+    if (c + 1 < BKV / 32)
+      ptx::tmem_ld_32x32b_x32(s_tmem + (c + 1) * 32, raw[(c + 1) & 1]);
+    sums.begin();
+#pragma unroll
+    for (int e = 0; e < 32; e += 4) {
+      float p[4];
+#pragma unroll
+      for (int i = 0; i < 4; i += 2) {
+        float r0, r1;
+        halves_of(fma2(pair_of(__uint_as_float(raw[c & 1][e + i]),
+                               __uint_as_float(raw[c & 1][e + i + 1])),
+                       scale2, negm2),
+                  r0, r1);
+        mx4[((e + i) >> 1) & 3] = max3(mx4[((e + i) >> 1) & 3], r0, r1);
+        p[i] = ex2(r0);
+        p[i + 1] = ex2(r1);
+        const __nv_bfloat162 pr = __floats2bfloat162_rn(p[i], p[i + 1]);
+        packed[c * 16 + ((e + i) >> 1)] = *reinterpret_cast<const uint32_t *>(&pr);
+      }
+      sums.add(e, p[0], p[1], p[2], p[3]);
+    }
+    sums.end(c, 1.0f);
+  }
+  rel_max = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+}
+
+/* probabilities_stored() with those sums. */
+__device__ __forceinline__ void
+probabilities_by64_stored(uint32_t s_tmem, float scale_log2, float neg_m, float fix,
+                          HalfSums &sums) {
+#pragma unroll 1
+  for (int c = 0; c < BKV / 32; c += 2) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t raw[32], packed[16];
+      ptx::tmem_ld_32x32b_x32(s_tmem + (c + h) * 32, raw);
+      ptx::tmem_ld_wait_for(raw);
+      sums.begin();
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        float p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          p[i] = ex2(fmaf(__uint_as_float(raw[e + i]), scale_log2, neg_m));
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(p[i], p[i + 1]);
+          packed[(e + i) >> 1] = *reinterpret_cast<const uint32_t *>(&pr);
+        }
+        sums.add(e, p[0], p[1], p[2], p[3]);
+      }
+      sums.end(h, c == 0 ? fix : 1.0f);
+      ptx::tmem_st_32x32b_x16(s_tmem + (c + h) * 16, packed);
+    }
+  }
+}
+
+/* The largest of `COLUMNS` scores of a row (as stored, before scaling). */
+template <int COLUMNS> __device__ __forceinline__ float row_max(uint32_t s_tmem) {
   float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll 1
-  for (int c = 0; c < BKV / 32; ++c) {
+  for (int c = 0; c < COLUMNS / 32; ++c) {
     uint32_t raw[32];
     ptx::tmem_ld_32x32b_x32(s_tmem + c * 32, raw);
     ptx::tmem_ld_wait_for(raw);
@@ -207,6 +303,7 @@ __device__ __forceinline__ void mask_scores(uint32_t s_tmem, int limit) {
     *stop = 1;                                                                 \
   } while (0)
 
+template <bool kBy64>
 __global__ void __launch_bounds__(THREADS, 1)
 flash_kernel(const __grid_constant__ CUtensorMap map_q,
               const __grid_constant__ CUtensorMap map_k,
@@ -437,7 +534,8 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
     const int n_mine = w ? n1 : n0;
     /* scores of unit-variance inputs stay within 2^8 of zero: start from a
        maximum of zero and let the check below catch what does not */
-    float m_used = 0.0f, l_sum = 0.0f;
+    float m_used = kBy64 ? -INFINITY : 0.0f, l_sum = 0.0f;
+    HalfSums halves;
     bool ok = true;
 
     for (int j = 0; ok && j < n_mine; ++j) {
@@ -461,14 +559,32 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
          memory, P has not been stored yet. (Written as a loop over two
          attempts, the compiler kept P live across the back edge and spilled:
          586 instead of 925 TFLOP/s.) */
-      probabilities(s_tmem, scale_log2, -m_used, packed, rel_max, sum);
-      const bool redo = __any_sync(0xffffffffu, rel_max > 8.0f ||
-                                                    (j == 0 && rel_max < -8.0f));
+      bool redo;
+      const HalfSums before = halves;
+      if (kBy64) {
+        if (j == 0) {
+          const float mx = row_max<64>(s_tmem) * scale_log2;
+          m_used = mx > m_used ? mx : m_used;
+        }
+        probabilities_by64(s_tmem, scale_log2, -m_used, packed, rel_max, halves);
+        /* a little below 8: what has grown is decided from the scores */
+        redo = __any_sync(0xffffffffu, rel_max > 7.99f);
+      } else {
+        probabilities(s_tmem, scale_log2, -m_used, packed, rel_max, sum);
+        redo = __any_sync(0xffffffffu, rel_max > 8.0f || (j == 0 && rel_max < -8.0f));
+      }
       if (redo) {
-        const float mx = row_max(s_tmem) * scale_log2;
-        const bool grow = mx > m_used + 8.0f || (j == 0 && mx < m_used - 8.0f);
-        const float m_new = grow ? mx : m_used;
-        const float fix = grow ? ex2(m_used - m_new) : 1.0f;
+        float m_new = m_used;
+        if (kBy64) {
+          const float m0 = row_max<64>(s_tmem) * scale_log2;
+          const float m1 = row_max<64>(s_tmem + 64) * scale_log2;
+          m_new = m0 > m_new + 8.0f ? m0 : m_new;
+          m_new = m1 > m_new + 8.0f ? m1 : m_new;
+        } else {
+          const float mx = row_max<BKV>(s_tmem) * scale_log2;
+          m_new = mx > m_used + 8.0f || (j == 0 && mx < m_used - 8.0f) ? mx : m_used;
+        }
+        const float fix = m_new != m_used ? ex2(m_used - m_new) : 1.0f;
         if (j > 0) {
           if (!ptx::mbar_wait(&bars->pv_done[w], (j - 1) & 1, stop)) {
             GIVE_UP(F2_PV_DONE);
@@ -488,9 +604,14 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
           }
           ptx::tmem_st_wait();
         }
-        l_sum *= fix;
         m_used = m_new;
-        sum = probabilities_stored(s_tmem, scale_log2, -m_used);
+        if (kBy64) {
+          halves = before;
+          probabilities_by64_stored(s_tmem, scale_log2, -m_used, fix, halves);
+        } else {
+          l_sum *= fix;
+          sum = probabilities_stored(s_tmem, scale_log2, -m_used);
+        }
       } else {
         /* P, two bf16 per column, over the first half of the score columns. */
         ptx::tmem_st_32x32b_x32(s_tmem,
@@ -511,7 +632,7 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
         GIVE_UP(F2_PV_DONE);
       } else {
         ptx::tc_fence_after_sync();
-        const float inv = 1.0f / l_sum;
+        const float inv = 1.0f / (kBy64 ? halves.l[0] + halves.l[1] : l_sum);
         __nv_bfloat16 *dst = out + ((int64_t)head_row + q_row) * HD;
 #pragma unroll 1
         for (int c = 0; c < HD / 32; ++c) {
@@ -566,13 +687,14 @@ const char *flash_attention_fwd(const void *q, const void *k, const void *v,
       !make_map_16(&mk, k, HD, rows, HD, 64, BKV, true) ||
       !make_map_16(&mv, v, HD, rows, HD, 64, BKV, true))
     return "cuTensorMapEncodeTiled refused q, k or v";
-  if (allow_dynamic_smem((const void *)flash_kernel, SMEM_BYTES) != cudaSuccess)
+  auto kernel = S % (BQ * NQ) ? flash_kernel<true> : flash_kernel<false>;
+  if (allow_dynamic_smem((const void *)kernel, SMEM_BYTES) != cudaSuccess)
     return "flash attention could not get its shared memory";
   const int64_t blocks = (int64_t)B * H * ((S / BQ + 1) / 2);
   if (blocks > INT32_MAX)
     return "flash attention is asked for too many tiles";
   const dim3 grid((unsigned)blocks);
-  flash_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(
+  kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(
       mq, mk, mv, (__nv_bfloat16 *)out, S, scale * 1.4426950408889634f,
       causal ? 1 : 0);
   const cudaError_t e = cudaGetLastError();
