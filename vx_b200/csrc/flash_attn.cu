@@ -14,13 +14,15 @@
  * Sequences of whole pairs of Q tiles start from a maximum of zero.  Those of an
  * odd number of tiles (kBy64) round as 64-key tiles do: their maximum starts as
  * that of a row's first 64 keys, and the row sums are kept in the same order.  The
- * two choices are equally far from 64 bits (2.33e-3 of bf16 rounding) and 3.2e-3
- * from each other; a sequence keeps the one its results have always had.
+ * two choices are 3e-3 from each other; the second is nearer to 64 bits under a
+ * causal mask (2.1e-3 and 2.3e-3 at 2176 positions; a row's first key has weight 1
+ * there) and as near without one, and a sequence keeps the one its results have
+ * always had.
  * [2, 32, 1152, 128] without a mask takes 69.3 us that way and 67.6 from a maximum
  * of zero; kernels of 64-key tiles took 88.2.
  *
- * A CTA owns two tiles of 128 query rows of one (batch, head), or the one that an
- * odd number of tiles leaves over, and walks KV tiles of 128 rows:
+ * A CTA owns two tiles of 128 query rows of one (batch, head), or a single one, and
+ * walks KV tiles of 128 rows:
  *   warp 0      TMA: the Q tiles once, then K and V tiles into rings;
  *   warp 1      issues tcgen05.mma, S = Q K^T and O += P V;
  *   warps 2..   one warpgroup per Q tile, one thread per query row.
@@ -37,6 +39,7 @@
  */
 #include "kernels.h"
 #include "launch.cuh"
+#include "launch_util.h"
 #include "ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -308,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 flash_kernel(const __grid_constant__ CUtensorMap map_q,
               const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v,
-              __nv_bfloat16 *__restrict__ out, int S, float scale_log2,
+              __nv_bfloat16 *__restrict__ out, int S, int pairs, float scale_log2,
               int causal) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
@@ -319,11 +322,11 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
   Bars *bars = reinterpret_cast<Bars *>(sm_v + RING * TILE_BYTES);
 
   const int warp = ptx::warp_index(), lane = threadIdx.x % 32;
-  /* A head is S / 256 pairs of Q tiles and, where S is an odd number of tiles, one
-     tile more. The single tiles come first where a later tile meets more keys, and last
-     where they are what is left over. Of a head's pairs the heavy ones come first. */
-  const int pairs = S / (BQ * NQ), heads = gridDim.x / ((S / BQ + 1) / 2);
-  const int singles = S % (BQ * NQ) ? heads : 0;
+  /* A head is `pairs` pairs of Q tiles and then single ones. Those come first where a
+     later tile meets more keys, and last where they are what is left over. Of a head's
+     pairs, and of the single tiles, the heavy ones come first. */
+  const int lone = S / BQ - pairs * NQ, heads = gridDim.x / (pairs + lone);
+  const int singles = heads * lone;
   int at = blockIdx.x, single = -1;
   if (causal && at < singles)
     single = at;
@@ -332,8 +335,9 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
   else if (at >= heads * pairs)
     single = at - heads * pairs;
   const bool two = single < 0;
-  const int head = two ? at / pairs : single;
-  const int q_base = (two ? pairs - 1 - at % pairs : pairs) * BQ * NQ;
+  const int head = two ? at / pairs : single % heads;
+  const int q_base = two ? (pairs - 1 - at % pairs) * BQ * NQ
+                         : (S / BQ - 1 - single / heads) * BQ;
   const int64_t head_row = (int64_t)head * S;
   /* KV tiles that Q tile 0 and Q tile 1 meet: n0 <= n1 <= n0 + 1, or n1 = 0. */
   const int n0 = causal ? q_base / BKV + 1 : S / BKV;
@@ -690,12 +694,16 @@ const char *flash_attention_fwd(const void *q, const void *k, const void *v,
   auto kernel = S % (BQ * NQ) ? flash_kernel<true> : flash_kernel<false>;
   if (allow_dynamic_smem((const void *)kernel, SMEM_BYTES) != cudaSuccess)
     return "flash attention could not get its shared memory";
-  const int64_t blocks = (int64_t)B * H * ((S / BQ + 1) / 2);
+  /* Of an odd number of tiles the last is alone; all are where each finds an SM of its
+     own: [1, 8, 640, 128] without a mask 14.4 us, 17.9 in pairs. */
+  const int64_t tiles = S / BQ;
+  const int pairs = tiles % 2 && B * H * tiles <= sm_count() ? 0 : (int)(tiles / 2);
+  const int64_t blocks = (int64_t)B * H * (tiles - pairs);
   if (blocks > INT32_MAX)
     return "flash attention is asked for too many tiles";
   const dim3 grid((unsigned)blocks);
   kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(
-      mq, mk, mv, (__nv_bfloat16 *)out, S, scale * 1.4426950408889634f,
+      mq, mk, mv, (__nv_bfloat16 *)out, S, pairs, scale * 1.4426950408889634f,
       causal ? 1 : 0);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
