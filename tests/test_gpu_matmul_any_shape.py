@@ -111,3 +111,15 @@ def test_16_bit_products_of_any_shape(oracle, dtype, m, n, k, off, pad):
     got = product(to(a), to(b), m, n, k, abi.BF16 if bf16 else abi.F16, bf16,
                   offsets=(off, off, off), pads=(pad, pad, pad))
     assert np.array_equal(got, to(exact))
+
+
+@pytest.mark.parametrize("k", [65, 128, 129, 193, 1025, 1088, 1537, 2100])
+def test_f32_products_whose_tiles_have_all_of_k(k):
+    """Eighty tiles: a block each, so that its two sets of accumulators alternate over the
+    whole of K, with a last segment of one block and of several."""
+    rng = np.random.default_rng(k)
+    m, n = 1280, 1021
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    assert rel(product(a, b, m, n, k, abi.F32), want) <= 6e-7

@@ -50,7 +50,7 @@ __device__ int g_tile_status; /* first wait that ran out since the last read */
 
 struct Bars {
   uint64_t full[STAGES], empty[STAGES];
-  uint64_t done, drained;
+  uint64_t done, drained[2]; /* drained: one for each set of accumulators */
   uint32_t tmem_base;
   int stop;
   int plain; /* a value was met that the split cannot carry */
@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
       ptx::mbar_init(&bars->empty[s], 1);
     }
     ptx::mbar_init(&bars->done, 1);
-    ptx::mbar_init(&bars->drained, LOADERS / 32);
+    for (int a = 0; a < 2; ++a)
+      ptx::mbar_init(&bars->drained[a], LOADERS / 32);
     bars->stop = 0;
     bars->plain = 0;
     ptx::fence_barrier_init();
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
       ptx::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0)
-        ptx::mbar_arrive(&bars->drained);
+        ptx::mbar_arrive(&bars->drained[seg & 1]);
       return true;
     };
     uint32_t lo = 0xffffffffu, hi = 0;
@@ -259,8 +260,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
       const int it = kb - kb0, s = it % STAGES;
       const int seg = it / kSegment;
       const bool first = it % kSegment == 0;
-      /* two sets of accumulators alternate */
-      if (first && seg > 1 && !ptx::mbar_wait_warp(&bars->drained, seg & 1, stop)) {
+      /* Two sets of accumulators alternate. Each has a barrier of its own: this warp may
+         come here so late that the segment before has been drained as well, and a shared
+         one would then be two phases on, which its parity does not tell from none. This
+         set's next phase is this segment's, so it cannot run ahead. */
+      if (first && seg > 1 &&
+          !ptx::mbar_wait_warp(&bars->drained[seg & 1], ((seg >> 1) - 1) & 1, stop)) {
         atomicCAS(&g_tile_status, 0, T_DRAINED);
         *stop = 1;
         break;
