@@ -123,3 +123,15 @@ def test_f32_products_whose_tiles_have_all_of_k(k):
     b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
     want = a.astype(np.float64) @ b.astype(np.float64)
     assert rel(product(a, b, m, n, k, abi.F32), want) <= 6e-7
+
+
+@pytest.mark.parametrize("m,n,k", [(1500, 1300, 1000), (1500, 1300, 130), (257, 300, 190)])
+def test_f32_products_of_one_sign(m, n, k):
+    """The tensor core cuts every sum off, so that values of one sign all lose: 2.2e-8 a K
+    step of 16, over the eight steps of a segment, and the f32 additions of the segments'
+    sums, which err to both sides (the FP32 pipe is 4.2e-7 off at 1000 of K)."""
+    rng = np.random.default_rng(k)
+    a = rng.uniform(0, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(0, 1, (k, n)).astype(np.float32)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    assert rel(product(a, b, m, n, k, abi.F32), want) <= 1.4 * 8 * 2.2e-8

@@ -41,7 +41,11 @@ constexpr int STAGE_BYTES = 6 * TERM_BYTES;
 constexpr int LOADERS = 512; /* threads that read, split and, at the end, add up */
 constexpr int THREADS = LOADERS + 32;
 constexpr int PITCH = BN + 4; /* floats between rows of the block's own sums */
-constexpr int kSegment = 8;   /* blocks of K between two transfers to registers */
+/* Blocks of K between two transfers to registers. The tensor core cuts its sums off
+   where an f32 addition rounds them: values of one sign lose 2.2e-8 a K step of 16. With
+   eight blocks 1500 x 1300 x 1000 of values in [0, 1) was 7.0e-7 off, on the FP32 pipe
+   4.2e-7; with two it is 1.4e-7, and 1024^3 takes 25.3 us instead of 25.2. */
+constexpr int kSegment = 2;
 constexpr uint32_t kSmallest = 0x09000000u; /* 2^-109 */
 constexpr uint32_t kLargest = 0x5d800000u;  /* 2^60 */
 
