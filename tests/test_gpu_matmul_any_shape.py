@@ -40,7 +40,7 @@ def rel(got, want):
     return np.linalg.norm(got.astype(np.float64) - want) / np.linalg.norm(want)
 
 
-# edges of the 128 x 128 x 64 tiles, of the eight-block segments (512 of K), of the runs
+# edges of the 128 x 128 x 64 tiles, of the two-block segments (128 of K), of the runs
 # that 2, 4 and 8 blocks of a cluster take, and views off the 16- and 8-byte grids
 F32 = [(1, 1, 1, 0, 0), (128, 128, 64, 0, 0), (129, 127, 65, 0, 0), (257, 300, 190, 2, 0),
        (130, 70, 513, 1, 3), (64, 64, 64 * 9, 0, 2), (100, 100, 64 * 17, 4, 4),
@@ -49,7 +49,7 @@ F32 = [(1, 1, 1, 0, 0), (128, 128, 64, 0, 0), (129, 127, 65, 0, 0), (257, 300, 1
 
 @pytest.mark.parametrize("m,n,k,off,pad", F32)
 def test_f32_products_of_any_shape(m, n, k, off, pad):
-    """The sums of 512 of K, in the tensor core, and their f32 total: within 1e-6 of an
+    """The sums of 128 of K, in the tensor core, and their f32 total: within 1e-6 of an
     f64 product (the f32 kernel's own bound in this suite is 2e-6), with values that differ
     by twelve orders of magnitude."""
     rng = np.random.default_rng(m + n + k)
@@ -135,3 +135,53 @@ def test_f32_products_of_one_sign(m, n, k):
     b = rng.uniform(0, 1, (k, n)).astype(np.float32)
     want = a.astype(np.float64) @ b.astype(np.float64)
     assert rel(product(a, b, m, n, k, abi.F32), want) <= 1.4 * 8 * 2.2e-8
+
+
+def microseconds(a, b, m, n, k):
+    """Of one product of device tensors, the least of five runs of twenty."""
+    import torch
+    ta, tb = abi.DeviceTensor.from_host(a), abi.DeviceTensor.from_host(b)
+    tc = abi.DeviceTensor.from_host(np.zeros((m, n), np.float32))
+    begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    runs = []
+    for _ in range(6):
+        begin.record()
+        for _ in range(20):
+            ops.matmul_into(tc, ta, tb)
+        end.record()
+        torch.cuda.synchronize()
+        runs.append(begin.elapsed_time(end) * 50)
+    for t in (ta, tb, tc):
+        t.free()
+    return min(runs[1:])
+
+
+def test_f32_values_near_the_smallest_cost_nothing():
+    """A softmax weight far below its row's maximum is a value near 1e-38: no reason for
+    another path. And a value too large for the terms costs its blocks the multiply-adds of
+    the FP32 pipe, which are ten times as many cycles as the products, half of it here."""
+    rng = np.random.default_rng(5)
+    m, n, k = 1000, 1000, 1000
+    a = rng.uniform(0, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(0, 1, (k, n)).astype(np.float32)
+    plain = microseconds(a, b, m, n, k)
+    a[a < 0.3] = 1e-38
+    a[a < 0.4] = 1e-45
+    assert microseconds(a, b, m, n, k) <= 1.3 * plain
+    a[0, 0] = 1e30
+    assert microseconds(a, b, m, n, k) <= 5 * plain
+
+
+def test_f32_values_of_every_size_that_terms_carry():
+    """Rows and columns from the smallest subnormal up: the terms are exact, so the bound is
+    that of ordinary values, and half the smallest subnormal where a result is one."""
+    rng = np.random.default_rng(6)
+    m, n, k = 150, 140, 300
+    a = rng.uniform(1, 2, (m, k)).astype(np.float32)
+    b = rng.uniform(-2, 2, (k, n)).astype(np.float32)
+    a = (a.astype(np.float64) * 2.0 ** np.linspace(-149, 8, m)[:, None]).astype(np.float32)
+    b = (b.astype(np.float64) * 2.0 ** np.linspace(-140, 8, n)[None, :]).astype(np.float32)
+    got = product(a, b, m, n, k, abi.F32)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    assert np.all(np.abs(got - want) <= 1e-6 * size + 8 * 2.0 ** -150)

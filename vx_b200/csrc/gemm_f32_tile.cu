@@ -18,15 +18,19 @@
  * distributed shared memory in run order, so the result does not depend on timing,
  * and no scratch is needed.
  *
- * Values the split cannot carry -- infinities, NaN, magnitudes from 2^60 on (whose
- * terms' products could overflow where the product's own sum does not) and non-zero
- * ones below 2^-109 (whose third term is below the smallest bf16) -- are noticed
- * while they are read; a block that met one computes its run with plain f32
- * multiply-adds instead, as gemm_f32 (gemm_simt.cu) would.
+ * Both operands are multiplied by 2^24 before they are split, which is exact, so that the
+ * smallest f32 value has three normal terms; the sums are multiplied by 2^-48.  (Without
+ * it a softmax weight below 2^-109 would lose its third term.)  Values that are then too
+ * large -- infinities, NaN, magnitudes whose products could overflow, from 2^34 on for
+ * 1024 of K -- are noticed while they are read; a block that met one computes its run with
+ * plain f32 multiply-adds as well, as gemm_f32 (gemm_simt.cu) would.  The price of one such
+ * value, which the slowest block pays: 257 x 300 x 190 takes 21 us instead of 14, 1000^3 97
+ * instead of 27 (on the FP32 pipe alone 31 and 118).
  */
 #include "kernels.h"
 #include "launch.cuh"
 #include "launch_util.h"
+#include "plain_tile.cuh"
 #include "ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -46,8 +50,7 @@ constexpr int PITCH = BN + 4; /* floats between rows of the block's own sums */
    eight blocks 1500 x 1300 x 1000 of values in [0, 1) was 7.0e-7 off, on the FP32 pipe
    4.2e-7; with two it is 1.4e-7, and 1024^3 takes 25.3 us instead of 25.2. */
 constexpr int kSegment = 2;
-constexpr uint32_t kSmallest = 0x09000000u; /* 2^-109 */
-constexpr uint32_t kLargest = 0x5d800000u;  /* 2^60 */
+constexpr float kUp = 0x1p24f, kDown = 0x1p-48f; /* of an operand, of a sum */
 
 enum { T_EMPTY = 0x81, T_FULL, T_DONE, T_DRAINED };
 __device__ int g_tile_status; /* first wait that ran out since the last read */
@@ -60,25 +63,22 @@ struct Bars {
   int plain; /* a value was met that the split cannot carry */
 };
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + (int)sizeof(Bars) + 64;
-static_assert(BM * PITCH * 4 <= STAGES * STAGE_BYTES, "the sums reuse the stages");
+static_assert((BM * PITCH + kPlainFloats) * 4 <= STAGES * STAGE_BYTES,
+              "the sums and the plain product reuse the stages");
+static_assert(LOADERS == kPlainThreads && BM == 128 && BN == 128, "plain_tile");
 
-/* Eight values as three words of four bf16 pairs; lo and hi take part in the range
-   check: the smallest and the largest magnitude met, as bit patterns, zero as the
-   largest. */
+/* Eight values, 2^24 of each, as three words of four bf16 pairs; most: the largest
+   magnitude met, as a bit pattern. */
 __device__ __forceinline__ uint32_t pack(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t *>(&v);
 }
-__device__ __forceinline__ void split8(const float (&v)[8], uint8_t *at, uint32_t &lo,
-                                       uint32_t &hi) {
+__device__ __forceinline__ void split8(const float (&v)[8], uint8_t *at, uint32_t &most) {
   uint32_t w[3][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float x = v[2 * j], y = v[2 * j + 1];
-    const uint32_t ux = __float_as_uint(x) & 0x7fffffffu;
-    const uint32_t uy = __float_as_uint(y) & 0x7fffffffu;
-    lo = min(lo, min(ux - 1u, uy - 1u));
-    hi = max(hi, max(ux, uy));
+    const float x = v[2 * j] * kUp, y = v[2 * j + 1] * kUp;
+    most = max(most, max(__float_as_uint(x) & 0x7fffffffu, __float_as_uint(y) & 0x7fffffffu));
     const uint32_t p1 = pack(x, y);
     const float rx = x - __uint_as_float(p1 << 16);
     const float ry = y - __uint_as_float(p1 & 0xffff0000u);
@@ -93,36 +93,14 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint8_t *at, uint32_
         make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
 }
 
-/* Eight consecutive values of a row, zero outside [0, cols) and where !inside.
-   vec: how many at a time the row's alignment allows, 4, 2 or 1. */
-__device__ __forceinline__ void read8(float (&v)[8], const float *row, int c, int cols,
-                                      bool inside, int vec) {
-  const bool whole = inside && c + 8 <= cols;
-  if (whole && vec == 4) {
-    const float4 a = *reinterpret_cast<const float4 *>(row + c);
-    const float4 b = *reinterpret_cast<const float4 *>(row + c + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else if (whole && vec == 2) {
-#pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      const float2 a = *reinterpret_cast<const float2 *>(row + c + e);
-      v[e] = a.x;
-      v[e + 1] = a.y;
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-      v[e] = inside && c + e < cols ? row[c + e] : 0.0f;
-  }
-}
-
 struct TileGemm {
   const float *a, *b;
   float *c;
   int64_t lda, ldb, ldc;
   int m, n, k, z; /* z: blocks that share a tile */
   int vec_a, vec_b, vec_c;
+  uint32_t too_large; /* bits of the first magnitude, times 2^24, whose products could
+                         overflow in a sum of k */
 };
 
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGemm g) {
@@ -214,7 +192,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
         ptx::mbar_arrive(&bars->drained[seg & 1]);
       return true;
     };
-    uint32_t lo = 0xffffffffu, hi = 0;
+    uint32_t most = 0;
     if (kb0 < kb1) {
       read_a(kb0);
       read_b(kb0);
@@ -240,12 +218,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
       /* each half's next values are asked for as soon as its registers are free */
 #pragma unroll
       for (int i = 0; i < 2; ++i) /* 64 rows further: the swizzle is the same */
-        split8(va[i], a_at + s * STAGE_BYTES + i * 64 * 128, lo, hi);
+        split8(va[i], a_at + s * STAGE_BYTES + i * 64 * 128, most);
       if (kb + 1 < kb1)
         read_a(kb + 1);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
-        split8(vb[i], b_at + s * STAGE_BYTES + i * 32 * 128, lo, hi);
+        split8(vb[i], b_at + s * STAGE_BYTES + i * 32 * 128, most);
       if (kb + 1 < kb1)
         read_b(kb + 1);
       ptx::fence_proxy_async_smem();
@@ -255,7 +233,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
     }
     if (ok && kb0 < kb1)
       drain((kb1 - kb0 - 1) / kSegment);
-    if (hi >= kLargest || lo < kSmallest - 1u)
+    if (most >= g.too_large)
       bars->plain = 1;
   } else {
     const uint32_t wide = ptx::idesc_f16(true, false, true, BM, 2 * BN);
@@ -308,31 +286,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
   __syncthreads();
   float *sums = reinterpret_cast<float *>(smem);
   if (bars->plain && warp < LOADERS / 32) {
-    /* 16 x 32 threads, 8 x 4 results each, ascending k: rare, so short rather than
-       fast */
+    const PlainTile t{g.a, g.b, g.lda, g.ldb, g.m, g.n, g.vec_a, g.vec_b};
+    plain_tile(t, row0, col0, kb0 * BK, min(kb1 * BK, g.k), tid, sums + BM * PITCH, acc);
     const int ty = tid / 32, tx = tid % 32;
-    const int k_end = min(kb1 * BK, g.k);
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      acc[i] = 0.0f;
-    for (int kk = kb0 * BK; kk < k_end; ++kk) {
-      float x[8], y[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = row0 + ty * 8 + i;
-        x[i] = r < g.m ? g.a[(int64_t)r * g.lda + kk] : 0.0f;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = col0 + tx * 4 + j;
-        y[j] = c < g.n ? g.b[(int64_t)kk * g.ldb + c] : 0.0f;
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[i * 4 + j] = fmaf(x[i], y[j], acc[i * 4 + j]);
-    }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       *reinterpret_cast<float4 *>(sums + (ty * 8 + i) * PITCH + tx * 4) =
@@ -342,7 +298,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
 #pragma unroll
     for (int j = 0; j < 32; j += 4)
       *reinterpret_cast<float4 *>(mine + j) =
-          make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+          make_float4(acc[j] * kDown, acc[j + 1] * kDown, acc[j + 2] * kDown,
+                      acc[j + 3] * kDown);
   }
   if (g.z > 1)
     ptx::cluster_sync_all();
@@ -454,6 +411,11 @@ const char *gemm_f32_tile(const float *a, int64_t lda, const float *b, int64_t l
   g.vec_a = vec(a, lda);
   g.vec_b = vec(b, ldb);
   g.vec_c = vec(c, ldc) == 4;
+  /* k products of two such values, as their terms add up to them, stay below 2^127 */
+  int log2_k = 0;
+  while (((int64_t)1 << log2_k) < k)
+    ++log2_k;
+  g.too_large = (uint32_t)(127 + (126 - log2_k) / 2) << 23;
   const int z = blocks_of_tile(m, n, k);
   g.z = z;
   if (allow_dynamic_smem((const void *)gemm_f32_tile_kernel, SMEM_BYTES) != cudaSuccess)
