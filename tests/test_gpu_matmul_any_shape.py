@@ -185,3 +185,23 @@ def test_f32_values_of_every_size_that_terms_carry():
     want = a.astype(np.float64) @ b.astype(np.float64)
     size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
     assert np.all(np.abs(got - want) <= 1e-6 * size + 8 * 2.0 ** -150)
+
+
+# shapes that the time model sends to the terms made beforehand: one run straight to C, and
+# twelve runs whose sums another kernel adds, to rows that begin anywhere
+BEFOREHAND = [(3072, 3072, 1024, 0, 0), (2944, 2944, 320, 0, 0), (128, 128, 8192, 0, 0),
+              (128, 132, 8192, 1, 3)]
+
+
+@pytest.mark.parametrize("m,n,k,off,pad", BEFOREHAND)
+def test_f32_products_of_terms_made_beforehand(m, n, k, off, pad):
+    """The small products are added first, so that what the tensor core cuts off at a K step
+    counts only in the k / 16 steps of the largest: 2.2e-8 each for values of one sign, a
+    little more where the sums walk."""
+    rng = np.random.default_rng(m + k)
+    for lowest in (-1, 0):
+        a = rng.uniform(lowest, 1, (m, k)).astype(np.float32)
+        b = rng.uniform(lowest, 1, (k, n)).astype(np.float32)
+        got = product(a, b, m, n, k, abi.F32, offsets=(off, off, off), pads=(pad, pad, pad))
+        want = a.astype(np.float64) @ b.astype(np.float64)
+        assert rel(got, want) <= 1e-6 + 3e-8 * k / 16
