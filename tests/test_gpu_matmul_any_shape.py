@@ -205,3 +205,26 @@ def test_f32_products_of_terms_made_beforehand(m, n, k, off, pad):
         got = product(a, b, m, n, k, abi.F32, offsets=(off, off, off), pads=(pad, pad, pad))
         want = a.astype(np.float64) @ b.astype(np.float64)
         assert rel(got, want) <= 1e-6 + 3e-8 * k / 16
+
+
+@pytest.mark.parametrize("m,n,k,off,pad", BEFOREHAND)
+def test_f32_terms_made_beforehand_of_values_they_cannot_carry(m, n, k, off, pad):
+    """Infinities, NaN and values whose products would overflow, in a few rows and columns;
+    a row near the smallest f32. As plain f32 multiply-adds give them."""
+    rng = np.random.default_rng(m + k + 1)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    a[3, 5], a[m - 1, k - 1] = np.inf, 1e25
+    b[9, 17], b[7, n - 2] = np.nan, -np.inf
+    a[20] = rng.uniform(1, 2, k) * 1e-38
+    got = product(a, b, m, n, k, abi.F32, offsets=(off, off, off), pads=(pad, pad, pad))
+    with np.errstate(all="ignore"):
+        want = (a.astype(np.float64) @ b.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want))
+    assert np.array_equal(np.isneginf(got), np.isneginf(want))
+    fine = np.isfinite(want)
+    size = np.sqrt((np.where(np.isfinite(a), a, 0).astype(np.float64) ** 2).sum(1))[:, None] * \
+        np.sqrt((np.where(np.isfinite(b), b, 0).astype(np.float64) ** 2).sum(0))[None, :]
+    off_by = np.abs(np.where(fine, got, 0).astype(np.float64) - np.where(fine, want, 0))
+    assert (off_by / size).max() <= 1e-6 + 3e-8 * k / 16

@@ -13,17 +13,40 @@
  * -- the small products first: the tensor core cuts its sum off at every K step of 16, by
  * 2.2e-8 of what the sum then is, so only the k / 16 steps of a1 b1 count.  With a1 b1
  * first 3072^3 in one run was 3.4e-5 off (2.0e-5 of values in [0, 1)), so it is 2.9e-6
- * (8.9e-6).
- * it runs on the CTA-pair kernel of the prefill (tcgen05.mma.cta_group::2,
+ * (8.9e-6).  It runs on the CTA-pair kernel of the prefill (tcgen05.mma.cta_group::2,
  * f32 partial sums per run of K', added in run order).
+ *
+ * The range is that of gemm_f32_tile.cu: both operands times 2^24, the sums times 2^-48,
+ * and a flag for each 128 rows of A and 128 columns of B in which a value was met that is
+ * too large then (infinities and NaN among them).  A last launch computes the tiles of
+ * flagged rows and columns with plain multiply-adds; where there is none it adds 1.3 us
+ * to the 289 of 3072^3.
  */
 #include "kernels.h"
 #include "launch.cuh"
+#include "launch_util.h"
+#include "plain_tile.cuh"
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 namespace vxb {
 namespace {
+
+constexpr float kUp = 0x1p24f, kDown = 0x1p-48f; /* of an operand, of a sum */
+constexpr int TILE = 128; /* rows, or columns, behind a flag */
+__device__ __forceinline__ uint32_t magnitude(float x) {
+  return __float_as_uint(x) & 0x7fffffffu;
+}
+/* bits of the first magnitude, times 2^24, whose products could overflow: k products of
+   two such values, as their terms add up to them, stay below 2^127 */
+uint32_t too_large(int64_t k) {
+  int log2_k = 0;
+  while (((int64_t)1 << log2_k) < k)
+    ++log2_k;
+  return (uint32_t)(127 + (126 - log2_k) / 2) << 23;
+}
 
 __device__ __forceinline__ void three_terms(float v, __nv_bfloat16 &t1,
                                             __nv_bfloat16 &t2, __nv_bfloat16 &t3) {
@@ -36,7 +59,8 @@ __device__ __forceinline__ void three_terms(float v, __nv_bfloat16 &t1,
 /* A' from A: one thread per eight consecutive values of a row (k is a
    multiple of 64), six 16-byte stores. */
 __global__ void __launch_bounds__(256)
-split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k) {
+split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k,
+               uint32_t limit, volatile int *flags) {
   chain_release();
   chain_wait();
   const int per_row = k / 8;
@@ -46,12 +70,14 @@ split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k) {
   const int64_t r = idx / per_row;
   const int c = (int)(idx - r * per_row) * 8;
   const float *src = a + r * lda + c;
-  uint32_t w1[4], w2[4], w3[4];
+  uint32_t w1[4], w2[4], w3[4], most = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     __nv_bfloat16 x1, x2, x3, y1, y2, y3;
-    three_terms(src[2 * j], x1, x2, x3);
-    three_terms(src[2 * j + 1], y1, y2, y3);
+    const float x = src[2 * j] * kUp, y = src[2 * j + 1] * kUp;
+    most = max(most, max(magnitude(x), magnitude(y)));
+    three_terms(x, x1, x2, x3);
+    three_terms(y, y1, y2, y3);
     w1[j] = (uint32_t)__bfloat16_as_ushort(x1) | (uint32_t)__bfloat16_as_ushort(y1) << 16;
     w2[j] = (uint32_t)__bfloat16_as_ushort(x2) | (uint32_t)__bfloat16_as_ushort(y2) << 16;
     w3[j] = (uint32_t)__bfloat16_as_ushort(x3) | (uint32_t)__bfloat16_as_ushort(y3) << 16;
@@ -59,6 +85,8 @@ split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k) {
   const uint4 t1 = make_uint4(w1[0], w1[1], w1[2], w1[3]);
   const uint4 t2 = make_uint4(w2[0], w2[1], w2[2], w2[3]);
   const uint4 t3 = make_uint4(w3[0], w3[1], w3[2], w3[3]);
+  if (most >= limit)
+    flags[r / TILE] = 1;
   __nv_bfloat16 *row = out + r * 6 * k + c;
   *reinterpret_cast<uint4 *>(row) = t3;
   *reinterpret_cast<uint4 *>(row + k) = t2;
@@ -71,7 +99,8 @@ split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k) {
 /* B' from B [k, n]: a block transposes a 32 x 32 tile through shared memory,
    so that B is read along n and B' written along k. */
 __global__ void __launch_bounds__(256)
-split_bt_kernel(__nv_bfloat16 *out, const float *b, int64_t ldb, int k, int n) {
+split_bt_kernel(__nv_bfloat16 *out, const float *b, int64_t ldb, int k, int n,
+                uint32_t limit, volatile int *flags) {
   __shared__ __nv_bfloat16 tile[3][32][34];
   chain_release();
   chain_wait();
@@ -79,8 +108,10 @@ split_bt_kernel(__nv_bfloat16 *out, const float *b, int64_t ldb, int k, int n) {
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5; /* 32 x 8 */
   for (int r = ty; r < 32; r += 8) {
     __nv_bfloat16 t1, t2, t3;
-    const float v = (k0 + r < k && n0 + tx < n) ? b[(int64_t)(k0 + r) * ldb + n0 + tx]
-                                                 : 0.0f;
+    const float v =
+        (k0 + r < k && n0 + tx < n) ? b[(int64_t)(k0 + r) * ldb + n0 + tx] * kUp : 0.0f;
+    if (magnitude(v) >= limit)
+      flags[n0 / TILE] = 1;
     three_terms(v, t1, t2, t3);
     tile[0][r][tx] = t1;
     tile[1][r][tx] = t2;
@@ -129,12 +160,40 @@ sum_runs_kernel(float *c, int64_t ldc, const float *partials, int splits, int m,
   }
 }
 
+/* The tiles whose rows or columns are flagged, again, with plain multiply-adds. */
+__global__ void __launch_bounds__(kPlainThreads, 1)
+plain_tiles_kernel(const PlainTile g, float *c, int64_t ldc, int k, const int *row_flags,
+                   const int *column_flags) {
+  extern __shared__ __align__(16) float room[];
+  chain_release();
+  chain_wait();
+  const int row_tiles = (g.m + TILE - 1) / TILE, column_tiles = (g.n + TILE - 1) / TILE;
+  for (int64_t t = blockIdx.x; t < (int64_t)row_tiles * column_tiles; t += gridDim.x) {
+    const int tm = (int)(t / column_tiles), tn = (int)(t - (int64_t)tm * column_tiles);
+    if (!row_flags[tm] && !column_flags[tn])
+      continue;
+    float acc[32];
+    plain_tile(g, tm * TILE, tn * TILE, 0, k, threadIdx.x, room, acc);
+    const int row = tm * TILE + threadIdx.x / 32 * 8, col = tn * TILE + threadIdx.x % 32 * 4;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (row + i / 4 < g.m && col + i % 4 < g.n)
+        c[(int64_t)(row + i / 4) * ldc + col + i % 4] = acc[i];
+    __syncthreads(); /* the next tile's first stage may be this one's last */
+  }
+}
+
+size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
+size_t flag_bytes(int64_t m, int64_t n) {
+  return up256((size_t)((m + TILE - 1) / TILE + (n + TILE - 1) / TILE) * sizeof(int));
+}
+
 bool direct(int splits, int64_t n, int64_t ldc) { return splits == 1 && ldc == n; }
 
 /* How many runs the K blocks are cut into: the number, up to 12, that leaves the
    last wave of pairs fullest. Many short runs rather than the fewest that are as
-   fast: the tensor core's own f32 sums lose a little with their length (1024^3 in
-   4 runs: relative error 2.2e-6, in 9: 9e-7). */
+   fast: the tensor core's own f32 sums lose a little with their length (1024^3 with
+   a1 b1 first in 4 runs: relative error 2.2e-6, in 9: 9e-7). */
 int runs_of(int64_t m, int64_t n, int64_t k) {
   const int tiles = (int)(((m + 255) / 256) * ((n + 255) / 256));
   const int k_blocks = (int)(6 * k / 64), pairs = 74;
@@ -168,8 +227,7 @@ size_t gemm_f32_split_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t ldc
       6 * k > (1ll << 31) - 1 || m * n * k < (1ll << 24))
     return 0;
   const int splits = runs_of(m, n, k);
-  size_t bytes = (size_t)(m + n) * 6 * k * 2;
-  bytes = (bytes + 255) & ~(size_t)255;
+  size_t bytes = flag_bytes(m, n) + up256((size_t)(m + n) * 6 * k * 2);
   if (!direct(splits, n, ldc))
     bytes += (size_t)splits * m * n * 4;
   return bytes;
@@ -180,20 +238,23 @@ const char *gemm_f32_split(const float *a, int64_t lda, const float *b, int64_t 
                            void *scratch, cudaStream_t stream) {
   if (!gemm_f32_split_scratch_bytes(m, n, k, ldc) || !scratch)
     return "the shape is not for the tensor-core f32 product";
-  __nv_bfloat16 *a6 = (__nv_bfloat16 *)scratch;
+  int *row_flags = (int *)scratch, *column_flags = row_flags + (m + TILE - 1) / TILE;
+  __nv_bfloat16 *a6 = (__nv_bfloat16 *)((char *)scratch + flag_bytes(m, n));
   __nv_bfloat16 *b6 = a6 + m * 6 * k;
-  const size_t terms_bytes = ((size_t)(m + n) * 6 * k * 2 + 255) & ~(size_t)255;
-  float *partials = (float *)((char *)scratch + terms_bytes);
+  float *partials = (float *)((char *)a6 + up256((size_t)(m + n) * 6 * k * 2));
+  const uint32_t limit = too_large(k);
+  if (cudaMemsetAsync(row_flags, 0, flag_bytes(m, n), stream) != cudaSuccess)
+    return "the flags of the f32 product could not be cleared";
   launch_chained(split_a_kernel, dim3((unsigned)((m * (k / 8) + 255) / 256)), dim3(256),
-                 0, stream, a6, a, lda, (int)m, (int)k);
+                 0, stream, a6, a, lda, (int)m, (int)k, limit, row_flags);
   launch_chained(split_bt_kernel, dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)),
-                 dim3(256), 0, stream, b6, b, ldb, (int)k, (int)n);
+                 dim3(256), 0, stream, b6, b, ldb, (int)k, (int)n, limit, column_flags);
   if (cudaGetLastError() != cudaSuccess)
     return "the term-splitting launches failed";
   int splits = runs_of(m, n, k);
   float *out = direct(splits, n, ldc) ? c : partials;
   if (const char *why = rows_gemm_of(a6, 6 * k, b6, 6 * k, (int)m, (int)n, out, &splits,
-                                     stream, splits))
+                                     stream, splits, kDown))
     return why;
   if (out != c) {
     const int vec = ldc % 4 == 0 && ((uintptr_t)c & 15) == 0;
@@ -202,6 +263,20 @@ const char *gemm_f32_split(const float *a, int64_t lda, const float *b, int64_t 
     if (cudaGetLastError() != cudaSuccess)
       return "the launch that adds the runs failed";
   }
+  constexpr int room = kPlainFloats * 4;
+  if (allow_dynamic_smem((const void *)plain_tiles_kernel, room) != cudaSuccess)
+    return "the plain tiles could not get their shared memory";
+  auto vec = [](const float *p, int64_t ld) {
+    return ((uintptr_t)p & 15) == 0 && ld % 4 == 0 ? 4
+           : ((uintptr_t)p & 7) == 0 && ld % 2 == 0 ? 2 : 1;
+  };
+  const int64_t tiles = ((m + TILE - 1) / TILE) * ((n + TILE - 1) / TILE);
+  launch_chained(plain_tiles_kernel, dim3((unsigned)std::min<int64_t>(tiles, sm_count())),
+                 dim3(kPlainThreads), room, stream,
+                 PlainTile{a, b, lda, ldb, (int)m, (int)n, vec(a, lda), vec(b, ldb)}, c, ldc,
+                 (int)k, (const int *)row_flags, (const int *)column_flags);
+  if (cudaGetLastError() != cudaSuccess)
+    return "the launch of the plain tiles failed";
   return nullptr;
 }
 

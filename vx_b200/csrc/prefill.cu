@@ -70,6 +70,7 @@ struct RowsGemm {
   int w_blocks;    /* of the weights: cols / 64 */
   int splits;
   float *partials; /* [splits][t][n] */
+  float scale;     /* of the sums */
 };
 
 /* Item -> (tile of positions, tile of weight rows, run). The runs and position
@@ -228,6 +229,9 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap map_x,
         uint32_t v[32];
         ptx::tmem_ld_32x32b_x32(taddr + c * 32, v);
         ptx::tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          v[e] = __float_as_uint(__uint_as_float(v[e]) * g.scale);
         if (row < g.t) {
           const int col = col0 + c * 32;
           if (col + 32 <= g.n) {
@@ -601,7 +605,7 @@ const char *rows_gemm(const void *terms, const void *w, int t, int n, int cols,
 
 const char *rows_gemm_of(const void *terms, int64_t term_cols, const void *w,
                          int64_t w_cols, int t, int n, float *partials,
-                         int *splits_out, cudaStream_t stream, int splits) {
+                         int *splits_out, cudaStream_t stream, int splits, float scale) {
   if (term_cols % BK != 0 || w_cols % BK != 0)
     return "the multi-position projections need columns in multiples of 64";
   if (allow_dynamic_smem((const void *)rows_gemm_kernel, SMEM_BYTES) != cudaSuccess)
@@ -618,6 +622,7 @@ const char *rows_gemm_of(const void *terms, int64_t term_cols, const void *w,
   g.w_blocks = (int)(w_cols / BK);
   g.splits = splits > 0 ? splits : rows_gemm_splits_of(t, n, term_cols);
   g.partials = partials;
+  g.scale = scale;
   *splits_out = g.splits;
   int pairs = resident_pairs();
   if (pairs < 1)
