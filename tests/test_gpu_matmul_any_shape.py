@@ -228,3 +228,23 @@ def test_f32_terms_made_beforehand_of_values_they_cannot_carry(m, n, k, off, pad
         np.sqrt((np.where(np.isfinite(b), b, 0).astype(np.float64) ** 2).sum(0))[None, :]
     off_by = np.abs(np.where(fine, got, 0).astype(np.float64) - np.where(fine, want, 0))
     assert (off_by / size).max() <= 1e-6 + 3e-8 * k / 16
+
+
+def test_f32_products_of_more_rows_than_tiles_in_a_grid():
+    """8.4 million rows: a shape with whole tiles goes where its rows fit."""
+    import torch
+    m, n, k = 65535 * 128 + 256, 128, 64
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    a = torch.rand((m, k), generator=g, device="cuda")
+    b = torch.rand((k, n), generator=g, device="cuda")
+    c = torch.zeros((m, n), device="cuda")
+    t = [abi.DeviceTensor(x.data_ptr(), tuple(x.shape), abi.F32, abi.home_gpu())
+         for x in (c, a, b)]
+    torch.cuda.synchronize()
+    ops.matmul_into(*t)
+    torch.cuda.synchronize()
+    for at in (0, 1 << 22, m - 300):
+        want = a[at:at + 300].double() @ b.double()
+        assert ((c[at:at + 300] - want).norm() / want.norm()).item() <= 1e-6
+    assert ops.kernel_status() == 0

@@ -35,6 +35,8 @@
 
 #include <cuda_bf16.h>
 
+#include <cmath>
+
 namespace vxb {
 namespace {
 
@@ -367,6 +369,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
   }
 }
 
+constexpr int64_t kMostRowTiles = 65535; /* in a grid's second dimension */
+
 /* How many blocks share a tile: more while the chip has room for them and each keeps
    a block of K. */
 int blocks_of_tile(int64_t m, int64_t n, int64_t k) {
@@ -385,6 +389,8 @@ int blocks_of_tile(int64_t m, int64_t n, int64_t k) {
    as many rounds as the tiles need. Measured 24.8 / 51.4 / 126 / 365 at 1024^3, 1536^3,
    2048^3, 3072^3, where this gives 21 / 52 / 128 / 371. */
 double gemm_f32_tile_us(int64_t m, int64_t n, int64_t k) {
+  if ((m + BM - 1) / BM > kMostRowTiles)
+    return HUGE_VAL;
   const int64_t z = blocks_of_tile(m, n, k);
   const int64_t blocks = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * z;
   const int64_t k_blocks = ((k + BK - 1) / BK + z - 1) / z;
@@ -398,7 +404,7 @@ const char *gemm_f32_tile(const float *a, int64_t lda, const float *b, int64_t l
     return nullptr;
   if (m > INT32_MAX - BM || n > INT32_MAX - BN || k > INT32_MAX - BK)
     return "a dimension does not fit in 32 bits";
-  if ((m + BM - 1) / BM > 65535)
+  if ((m + BM - 1) / BM > kMostRowTiles)
     return "more than 65535 row tiles";
   TileGemm g{};
   g.a = a; g.b = b; g.c = c;
