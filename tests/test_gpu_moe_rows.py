@@ -395,3 +395,52 @@ def test_fp8_product_unpacks_every_code(oracle):
     for j in range(0, cols, 5):
         want = oracle.quant_dot_f64("fp8", words, s, x[j], rows, cols)
         assert np.array_equal(got[j], want), j
+
+
+@pytest.mark.parametrize("align", [8, 16])
+@pytest.mark.parametrize("counts,inter,hidden", [
+    ([128, 120, 97, 113], 320, 320),          # whole segments; 48 columns of a set
+    ([0, 2, 500, 8, 38], 448, 384),           # nobody, a pair or two, hundreds; 7 and 6 blocks
+    ([700, 0, 600], 2496, 2624),              # more items than SMs; 39 and 41 blocks, 32 bits
+    ([513, 129, 640, 6], 2560, 2560)])        # of scales at a time; 40 blocks, 128 bits
+def test_grouped_experts_of_any_share(oracle, counts, inter, hidden, align):
+    """Experts of given numbers of pairs: segments up to full, blocks that go from item to
+    item. Pairs of every expert and tokens are checked against f64 loops as above."""
+    experts, k, pairs = len(counts), 2, sum(counts)
+    n = pairs // k
+    rng = np.random.default_rng(pairs + align)
+    ids = rng.permutation(np.repeat(np.arange(experts), counts)).astype(np.int32)
+    weights = rng.uniform(0.1, 1, (n, k)).astype(np.float32)
+    gu, gu_s = oracle.quant_inputs("q4", experts * 2 * inter, hidden, 31)
+    dn, dn_s = oracle.quant_inputs("q4", experts * hidden, inter, 33)
+    x = oracle.random_f32(n * hidden, 35, 1.0).reshape(n, hidden)
+    y0 = oracle.random_f32(n * hidden, 36, 1.0).reshape(n, hidden)
+    room = pairs + experts * (align - 1)
+    order, tile_expert = empty((room,)), empty(((room + align - 1) // align,))
+    blocks = (pairs + 255) // 256
+    ops.nn_moe_group(order, empty((blocks, experts)), empty((blocks, experts)),
+                     empty((experts + 1,)), tile_expert, dev(ids), experts, align)
+    mid, ty = dev(np.full((pairs, inter), np.nan, np.float32)), dev(y0)
+    ops.moe_swiglu_q4_grouped(mid, dev(gu), dev(gu_s), order, tile_expert, align, dev(x), n,
+                              k, inter, hidden, experts)
+    ops.moe_down_q4_add_grouped(ty, dev(dn), dev(dn_s), order, tile_expert, align,
+                                dev(weights.ravel()), mid,
+                                dev(np.full((pairs, hidden), np.nan, np.float32)), n, k,
+                                hidden, inter, experts)
+    mid, y = mid.to_host(), ty.to_host()
+    assert ops.kernel_status() == 0
+    assert np.isfinite(mid).all() and np.isfinite(y).all()
+    first = [int(np.argmax(ids == e)) for e in range(experts) if counts[e]]
+    last = [pairs - 1 - int(np.argmax(ids[::-1] == e)) for e in range(experts) if counts[e]]
+    for t in sorted({p // k for p in first + last + [int(rng.integers(pairs))]}):
+        gate_up = oracle.quant_dot_f64("q4", gu, gu_s, x[t], experts * 2 * inter, hidden)
+        want_y = y0[t].astype(np.float64)
+        for e in range(k):
+            pair = t * k + e
+            at = ids[pair] * 2 * inter
+            g, u = gate_up[at:at + inter], gate_up[at + inter:at + 2 * inter]
+            close(mid[pair], g / (1.0 + np.exp(-g)) * u)
+            down = oracle.quant_dot_f64("q4", dn, dn_s, mid[pair], experts * hidden, inter)
+            want_y += float(weights[t, e]) * down[ids[pair] * hidden:
+                                                  (ids[pair] + 1) * hidden]
+        close(y[t], want_y)

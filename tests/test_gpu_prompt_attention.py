@@ -58,3 +58,24 @@ def test_whole_cache(q_heads, kv_heads):
     many.close()
     del held, held_too
     assert ops.kernel_status() == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,window,rows", [(2, 1, 70, 129), (4, 2, 1000, 460)])
+def test_values_that_terms_cannot_carry(heads, kv_heads, window, rows):
+    """Keys of about 2^58 in a column that no query looks at and the output matrix scales
+    down: the logits are those of ordinary keys, by plain multiply-adds over the ring, with
+    the window and the gate."""
+    cfg = models_of.config(128, 96, [models_of.layer(heads, kv_heads, 128, window, 0.09, 64)])
+    w = models_of.weights(cfg, seed=window)
+    column = 37
+    w["l0.mix.q"].reshape(heads, 128, -1)[:, column] = 0.0
+    w["l0.mix.k"].reshape(kv_heads, 128, -1)[:, column] *= 2.0 ** 58
+    w["l0.mix.o"].reshape(-1, heads, 128)[:, :, column] *= 2.0 ** -58
+    tokens = tokens_for(cfg, 460)
+    want = plain.logits(tokens, w, cfg)
+    d = decoder(cfg, w, max_seq=460, prefill_rows=rows)
+    for sizes in ([rows], [2 * rows + 3, 1, 40]):
+        d.reset()
+        close(feed_all(d, tokens, cut(460, sizes)), want)
+    d.close()
+    assert ops.kernel_status() == 0
