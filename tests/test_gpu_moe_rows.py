@@ -10,12 +10,17 @@ kernel's, and within the reference's criterion of f64 loops. The grouped expert
 projections (vx_b200_moe_*_grouped) and the Q4_0 / fp8 products of many rows
 (vx_b200_gemm_q4, vx_b200_gemm_fp8) against f64 loops by the same criterion, max
 |got - want| <= 1e-5 * max |want|."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 from vx_b200 import abi, ops
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def dev(a, bf16=False):
@@ -444,3 +449,40 @@ def test_grouped_experts_of_any_share(oracle, counts, inter, hidden, align):
             want_y += float(weights[t, e]) * down[ids[pair] * hidden:
                                                   (ids[pair] + 1) * hidden]
         close(y[t], want_y)
+
+
+KEEPS = """
+import torch
+from vx_b200 import abi, ops
+inter, hidden = 1024, 2048
+def tensor(t, elem):
+    return abi.DeviceTensor(t.data_ptr(), tuple(t.shape), elem, abi.home_gpu())
+def zeros(shape, dtype):
+    return torch.zeros(shape, dtype=dtype, device="cuda")
+w, s = zeros((2 * inter, hidden // 8), torch.int32), zeros((2 * inter, hidden // 32), torch.float16)
+x, out = zeros((2000, hidden), torch.float32), zeros((2000, inter), torch.float32)
+def call(n):
+    # one expert: its pairs in order, in tiles of eight, and a tile of none
+    order, tiles = torch.full((n + 8,), -1, dtype=torch.int32, device="cuda"), zeros(n // 8 + 1, torch.int32)
+    order[:n] = torch.arange(n)
+    tiles[-1] = -1
+    ops.moe_swiglu_q4_grouped(tensor(out, abi.F32), tensor(w, abi.I32), tensor(s, abi.F16), tensor(order, abi.I32),
+                              tensor(tiles, abi.I32), 8, tensor(x, abi.F32), n, 1, inter, hidden, 1)
+    assert ops.kernel_status() == 0
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+print((call(8) - call(2000)) >> 20)
+"""
+
+
+@pytest.mark.parametrize("limit,kept", [("0", False), (None, True)])
+def test_what_the_experts_keep_of_their_scratch(limit, kept):
+    """2000 rows of 2048 as three bf16 terms, 24 MB: given back where
+    VX_CUDA_POOL_MAX_MB says to keep nothing."""
+    env = {k: v for k, v in os.environ.items() if k != "VX_CUDA_POOL_MAX_MB"}
+    if limit is not None:
+        env["VX_CUDA_POOL_MAX_MB"] = limit
+    out = subprocess.run([sys.executable, "-c", KEEPS], env=env, capture_output=True,
+                         text=True, timeout=300, cwd=ROOT)
+    assert out.returncode == 0, out.stderr[-800:]
+    assert (int(out.stdout.split()[-1]) >= 20) == kept, out.stdout

@@ -258,9 +258,9 @@ std::mutex g_on_stream_mu;
 std::unordered_map<void *, cudaStream_t> g_on_stream; /* cudaMallocAsync'd */
 
 /* Stream-ordered temporaries come from a pool of this library's own, one per
-   device, that keeps what is freed (the default pool gives its memory back to
-   the driver at the next synchronisation, and a product that needs 100 MB of
-   scratch on every call then pays for the allocation every time). */
+   device, that keeps what is freed, as much as VX_CUDA_POOL_MAX_MB says (the default
+   pool gives its memory back to the driver at the next synchronisation, and a product
+   that needs 100 MB of scratch on every call then pays for the allocation every time). */
 cudaMemPool_t stream_pool() {
   static std::mutex mu;
   static cudaMemPool_t pools[64] = {};
@@ -279,7 +279,7 @@ cudaMemPool_t stream_pool() {
       cudaGetLastError();
       return nullptr;
     }
-    uint64_t keep = UINT64_MAX;
+    uint64_t keep = vx::vx_pool_capacity_bytes();
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     pools[dev] = pool;
   }

@@ -704,8 +704,8 @@ size_t q4_tiles_scratch_bytes(const MoeGroupedArgs &m);
 const char *q4_tiles_grouped(const MoeGroupedArgs &m, bool swiglu, void *scratch,
                              cudaStream_t stream);
 int q4_tiles_status();
-/* Device memory until the end of a C++ scope, in stream order; ptr is null where there
-   was none (dispatch.cu). */
+/* Device memory until the end of a C++ scope, in stream order, from the current GPU's pool;
+   ptr is null where there was none (dispatch.cu). */
 class StreamScratch {
 public:
   explicit StreamScratch(size_t bytes);
