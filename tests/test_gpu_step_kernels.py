@@ -62,3 +62,33 @@ def test_blocks_per_head_do_not_change_the_logits(batch, q_heads, kv_heads):
     one.close()
     many.close()
     del held, held_too
+
+
+@pytest.mark.parametrize("batch,q_heads,kv_heads", [(4, 32, 32), (8, 32, 32), (16, 32, 32),
+                                                    (16, 64, 16)])
+def test_blocks_per_head_over_a_long_cache(batch, q_heads, kv_heads):
+    """The same keys and values for every sequence, 1500 positions: a block goes round its
+    loop of loads many times. Sums of 1500 weights in another order: 2^-24 a term at most,
+    and the terms add up to one."""
+    import torch
+    held, rows = 1500, 1536
+    shape = dict(dim=q_heads * 128, hidden=256, n_layers=1, q_heads=q_heads, kv_heads=kv_heads,
+                 head_dim=128, vocab=512, max_seq=rows)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(q_heads)
+    cache = [torch.randn((1, 1, rows, kv_heads, 128), generator=g, device="cuda")
+             for _ in range(2)]
+    got = []
+    for b in (1, batch):
+        d, weights = llama.nn_bf16_model(batch=b, **shape)
+        k, v = (c.expand(1, b, -1, -1, -1).contiguous() for c in cache)
+        torch.cuda.synchronize()
+        d.adopt_kv(k.data_ptr(), v.data_ptr(), held)
+        for step in range(3):
+            d.step([step + 1] * b)
+        got.append(d.logits())
+        d.close()
+        del weights
+    scale = np.sqrt((got[0] ** 2).mean())
+    assert np.abs(got[1] - got[0]).max() <= 1500 * 2.0 ** -24 * scale
+    assert ops.kernel_status() == 0

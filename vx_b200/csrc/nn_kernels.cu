@@ -547,6 +547,36 @@ size_t attn_scratch_floats(int batch, int q_heads, int head_dim, int max_seq,
          (head_dim + 2);
 }
 
+/* How many clusters of `cl` blocks the current GPU holds at once. */
+static int resident_clusters(const void *kernel, int cl, int threads) {
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, int> asked;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_pair(kernel, dev);
+  const auto hit = asked.find(key);
+  if (hit != asked.end())
+    return hit->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(threads);
+  cfg.gridDim = dim3(cl);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  asked[key] = n;
+  return n;
+}
+
 const char *attention_decode(const AttnArgs &a, cudaStream_t stream) {
   if (a.head_dim % 4 != 0 || a.head_dim > 128)
     return "head_dim must be a multiple of 4, and at most 128";
@@ -569,40 +599,55 @@ const char *attention_decode(const AttnArgs &a, cudaStream_t stream) {
   if (which != kAttnCluster && which != kAttnSplit)
     return "unknown attention kernel";
   if (which == kAttnCluster) {
-    /* Blocks per head: eight, or fewer where the heads of all sequences alone put a
-       block on most SMs: a block that starts, meets its cluster and leaves for a
-       handful of positions costs more than it reads (16 sequences of 32 heads at
-       position 120: 40 us a layer with eight blocks each, 63 MB of cache). */
     const int64_t heads = (int64_t)a.kv_heads * tiles * a.batch;
-    const int cl = heads <= 64 ? 8 : heads <= 128 ? 4 : heads <= 256 ? 2 : 1;
-    const dim3 cgrid(cl, a.kv_heads * tiles, a.batch);
-    /* Warps per block by how many blocks there are: with few heads (a rank of
-       a tensor-parallel job holds 4 or 8 of 32) sixteen warps per block put
-       the positions of a head on 128 warps, one round trip to memory each;
-       with every SM already holding several blocks, four. Measured at
-       position 520 on one rank's share of the 7B shape, microseconds per
-       layer for 4 / 8 / 16 warps: 1/2 of the heads 53.4 / 51.8 / 54.3, 1/4
-       37.7 / 37.3 / 36.0, 1/8 28.6 / 27.3 / 26.5; all heads 387 / 389 / 361
-       tokens/s. */
-    const int64_t blocks = heads * cl;
-    int warps = cl < 8 ? 4 : 2 * blocks <= sm_count() ? 16 : (blocks <= 2 * sm_count() ? 8 : 4);
-    /* VXB_ATTN_WARPS=4, 8 or 16 pins it (for measurements) */
-    if (const char *pin = getenv("VXB_ATTN_WARPS")) {
-      const int v = atoi(pin);
-      if (cl == 8 && (v == 4 || v == 8 || v == 16))
-        warps = v;
-    }
-    auto go = [&](auto kernel) {
-      launch_chained_cluster(kernel, cgrid, dim3(warps * 32), cl, stream, a);
+    /* Warps per block, with eight blocks a head, by how many blocks there are: with few
+       heads (a rank of a tensor-parallel job holds 4 or 8 of 32) sixteen warps per block
+       put the positions of a head on 128 warps, one round trip to memory each; with every
+       SM already holding several blocks, four. Measured at position 520 on one rank's
+       share of the 7B shape, microseconds per layer for 4 / 8 / 16 warps: 1/2 of the heads
+       53.4 / 51.8 / 54.3, 1/4 37.7 / 37.3 / 36.0, 1/8 28.6 / 27.3 / 26.5; all heads 387 /
+       389 / 361 tokens/s. */
+    int warps = 16 * heads <= sm_count() ? 16 : 4 * heads <= sm_count() ? 8 : 4;
+    /* VXB_ATTN_WARPS=4, 8 or 16 pins it, and the eight blocks (for measurements) */
+    const char *pin = getenv("VXB_ATTN_WARPS");
+    const int pinned = pin ? atoi(pin) : 0;
+    const bool is_pinned = pinned == 4 || pinned == 8 || pinned == 16;
+    if (is_pinned)
+      warps = pinned;
+    auto go = [&](auto kernel, int cl, int w) {
+      launch_chained_cluster(kernel, dim3(cl, a.kv_heads * tiles, a.batch), dim3(w * 32), cl,
+                             stream, a);
+    };
+    /* Fewer than eight blocks a head, of four warps, where that makes one wave of at least
+       three blocks an SM, or where the positions are few: a block that starts, meets its
+       cluster and leaves for a handful of them costs more than it reads. 16 sequences of 32
+       heads at position 120: 40 us a layer with eight blocks a head, 63 MB of cache; eight
+       of 32 at 1500, eight steps of four layers: 6.66 ms with eight blocks a head, 6.28
+       with two. What is more or less than one wave leaves SMs idle while the last blocks
+       read a long cache: four sequences of 36 heads at 3500 positions 11.26 ms with two
+       blocks a head, 10.84 with four, 9.84 with eight; 16 of 24 at 2000 9.38 with two and
+       8.88 with eight. (16 of 64 at 1000 are the exception: 15.2 with one, 15.8 with
+       eight.) */
+    auto few = [&](auto kernel, int cl) {
+      return !is_pinned &&
+             ((a.max_pos < 512 && heads * cl >= 512) ||
+              (heads * cl >= 3 * sm_count() &&
+               heads <= resident_clusters((const void *)kernel, cl, 4 * 32)));
     };
     auto of_heads = [&](auto gh_c) {
       constexpr int GH = decltype(gh_c)::value;
-      if (cl == 1) go(attention_cluster_kernel<GH, 4, 1>);
-      else if (cl == 2) go(attention_cluster_kernel<GH, 4, 2>);
-      else if (cl == 4) go(attention_cluster_kernel<GH, 4, 4>);
-      else if (warps == 16) go(attention_cluster_kernel<GH, 16, 8>);
-      else if (warps == 8) go(attention_cluster_kernel<GH, 8, 8>);
-      else go(attention_cluster_kernel<GH, 4, 8>);
+      if (few(attention_cluster_kernel<GH, 4, 1>, 1))
+        go(attention_cluster_kernel<GH, 4, 1>, 1, 4);
+      else if (few(attention_cluster_kernel<GH, 4, 2>, 2))
+        go(attention_cluster_kernel<GH, 4, 2>, 2, 4);
+      else if (few(attention_cluster_kernel<GH, 4, 4>, 4))
+        go(attention_cluster_kernel<GH, 4, 4>, 4, 4);
+      else if (warps == 16)
+        go(attention_cluster_kernel<GH, 16, 8>, 8, 16);
+      else if (warps == 8)
+        go(attention_cluster_kernel<GH, 8, 8>, 8, 8);
+      else
+        go(attention_cluster_kernel<GH, 4, 8>, 8, 4);
     };
     if (gh == 4) of_heads(std::integral_constant<int, 4>());
     else if (gh == 2) of_heads(std::integral_constant<int, 2>());
