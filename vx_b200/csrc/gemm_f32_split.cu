@@ -11,7 +11,7 @@
  *   A' [m, 6k] = a3 | a2 | a1 | a2 | a1 | a1
  *   B' [n, 6k] = b1 | b2 | b3 | b1 | b2 | b1      (B transposed on the way)
  * -- the small products first: the tensor core cuts its sum off at every K step of 16, by
- * 2.2e-8 of what the sum then is, so only the k / 16 steps of a1 b1 count.  With a1 b1
+ * up to 2^-24 of what the sum then is, so only the k / 16 steps of a1 b1 count.  With a1 b1
  * first 3072^3 in one run was 3.4e-5 off (2.0e-5 of values in [0, 1)), so it is 2.9e-6
  * (8.9e-6).  It runs on the CTA-pair kernel of the prefill (tcgen05.mma.cta_group::2,
  * f32 partial sums per run of K', added in run order).
@@ -36,6 +36,13 @@ namespace {
 
 constexpr float kUp = 0x1p24f, kDown = 0x1p-48f; /* of an operand, of a sum */
 constexpr int TILE = 128; /* rows, or columns, behind a flag */
+/* Where values too large for the terms were met. split_bt leaves a word for each of its
+   blocks and clears the rows' words; split_a, after it, sets those and gathers the others. */
+struct Flags {
+  int *rows, *columns; /* for each TILE of them */
+  int *blocks;         /* [down][across]: of 32 x 32 values of B */
+  int row_tiles, down, across;
+};
 __device__ __forceinline__ uint32_t magnitude(float x) {
   return __float_as_uint(x) & 0x7fffffffu;
 }
@@ -57,12 +64,25 @@ __device__ __forceinline__ void three_terms(float v, __nv_bfloat16 &t1,
 }
 
 /* A' from A: one thread per eight consecutive values of a row (k is a
-   multiple of 64), six 16-byte stores. */
+   multiple of 64), six 16-byte stores. The last blocks gather the flags that split_bt's
+   blocks left, one block for each 128 columns. */
 __global__ void __launch_bounds__(256)
 split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k,
-               uint32_t limit, volatile int *flags) {
+               uint32_t limit, const Flags f) {
   chain_release();
   chain_wait();
+  const int gatherers = (f.across + 3) / 4;
+  const int column = (int)blockIdx.x - (int)gridDim.x + gatherers;
+  if (column >= 0) {
+    int any = 0;
+    for (int i = threadIdx.x; i < 4 * f.down; i += blockDim.x)
+      if (4 * column + i % 4 < f.across)
+        any |= f.blocks[i / 4 * f.across + 4 * column + i % 4];
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0)
+      f.columns[column] = any;
+    return;
+  }
   const int per_row = k / 8;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)m * per_row)
@@ -86,7 +106,7 @@ split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k,
   const uint4 t2 = make_uint4(w2[0], w2[1], w2[2], w2[3]);
   const uint4 t3 = make_uint4(w3[0], w3[1], w3[2], w3[3]);
   if (most >= limit)
-    flags[r / TILE] = 1;
+    f.rows[r / TILE] = 1;
   __nv_bfloat16 *row = out + r * 6 * k + c;
   *reinterpret_cast<uint4 *>(row) = t3;
   *reinterpret_cast<uint4 *>(row + k) = t2;
@@ -100,24 +120,29 @@ split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k,
    so that B is read along n and B' written along k. */
 __global__ void __launch_bounds__(256)
 split_bt_kernel(__nv_bfloat16 *out, const float *b, int64_t ldb, int k, int n,
-                uint32_t limit, volatile int *flags) {
+                uint32_t limit, const Flags f) {
   __shared__ __nv_bfloat16 tile[3][32][34];
   chain_release();
   chain_wait();
   const int k0 = blockIdx.y * 32, n0 = blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5; /* 32 x 8 */
+  int large = 0;
   for (int r = ty; r < 32; r += 8) {
     __nv_bfloat16 t1, t2, t3;
     const float v =
         (k0 + r < k && n0 + tx < n) ? b[(int64_t)(k0 + r) * ldb + n0 + tx] * kUp : 0.0f;
-    if (magnitude(v) >= limit)
-      flags[n0 / TILE] = 1;
+    large |= magnitude(v) >= limit;
     three_terms(v, t1, t2, t3);
     tile[0][r][tx] = t1;
     tile[1][r][tx] = t2;
     tile[2][r][tx] = t3;
   }
-  __syncthreads();
+  large = __syncthreads_or(large);
+  if (threadIdx.x == 0)
+    f.blocks[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = large;
+  for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+       i < f.row_tiles; i += (int64_t)gridDim.x * gridDim.y * blockDim.x)
+    f.rows[i] = 0;
   for (int j = ty; j < 32; j += 8) {
     if (n0 + j >= n || k0 + tx >= k)
       continue;
@@ -184,8 +209,20 @@ plain_tiles_kernel(const PlainTile g, float *c, int64_t ldc, int k, const int *r
 }
 
 size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
-size_t flag_bytes(int64_t m, int64_t n) {
-  return up256((size_t)((m + TILE - 1) / TILE + (n + TILE - 1) / TILE) * sizeof(int));
+Flags flags_of(void *at, int64_t m, int64_t n, int64_t k) {
+  Flags f;
+  f.row_tiles = (int)((m + TILE - 1) / TILE);
+  f.down = (int)((k + 31) / 32);
+  f.across = (int)((n + 31) / 32);
+  f.rows = (int *)at;
+  f.columns = f.rows + f.row_tiles;
+  f.blocks = f.columns + (n + TILE - 1) / TILE;
+  return f;
+}
+size_t flag_bytes(int64_t m, int64_t n, int64_t k) {
+  const Flags f = flags_of(nullptr, m, n, k);
+  return up256((size_t)(f.row_tiles + (n + TILE - 1) / TILE + (int64_t)f.down * f.across) *
+               sizeof(int));
 }
 
 bool direct(int splits, int64_t n, int64_t ldc) { return splits == 1 && ldc == n; }
@@ -212,13 +249,18 @@ int runs_of(int64_t m, int64_t n, int64_t k) {
 
 } // namespace
 
-/* Microseconds, about: the six products at 1.5 PFLOP/s, the terms (12 bytes a value)
-   and the runs' partial sums (8) written and read, four launches. Measured 39.5 / 61.5 /
-   154 / 288 at 1024^3, 1536^3, 2048^3, 3072^3, where this gives 48 / 65 / 171 / 292. */
+/* Microseconds, about: the six products at 1.5 PFLOP/s, or 0.34 for a block of K' of each
+   pair's items where there are few, the terms (12 bytes a value) and the runs' partial sums
+   (8) written and read, five launches. Measured 154 / 105 / 290 / 40.6 at 2048^3, 3072 x
+   3072 x 1024, 3072^3 and 128 x 128 x 8192, where this gives 174 / 110 / 295 / 45. */
 double gemm_f32_split_us(int64_t m, int64_t n, int64_t k, int64_t ldc) {
-  const int runs = runs_of(m, n, k);
-  const double sums = direct(runs, n, ldc) ? 0.0 : 8.0e-6 * runs * m * n / 4.0;
-  return 15.0 + 12.0e-9 * m * n * k / 1.5 + 24.0e-6 * (m + n) * k / 10.0 + sums;
+  const int64_t runs = runs_of(m, n, k), pairs = 74;
+  const int64_t items = (m + 255) / 256 * ((n + 255) / 256) * runs;
+  const double sums = direct((int)runs, n, ldc) ? 0.0 : 8.0e-6 * runs * m * n / 4.0;
+  const double longest =
+      0.34 * (double)((items + pairs - 1) / pairs * ((6 * k / 64 + runs - 1) / runs));
+  return 18.0 + std::max(12.0e-9 * m * n * k / 1.5, longest) + 24.0e-6 * (m + n) * k / 10.0 +
+         sums;
 }
 
 size_t gemm_f32_split_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t ldc) {
@@ -227,7 +269,7 @@ size_t gemm_f32_split_scratch_bytes(int64_t m, int64_t n, int64_t k, int64_t ldc
       6 * k > (1ll << 31) - 1 || m * n * k < (1ll << 24))
     return 0;
   const int splits = runs_of(m, n, k);
-  size_t bytes = flag_bytes(m, n) + up256((size_t)(m + n) * 6 * k * 2);
+  size_t bytes = flag_bytes(m, n, k) + up256((size_t)(m + n) * 6 * k * 2);
   if (!direct(splits, n, ldc))
     bytes += (size_t)splits * m * n * 4;
   return bytes;
@@ -238,17 +280,16 @@ const char *gemm_f32_split(const float *a, int64_t lda, const float *b, int64_t 
                            void *scratch, cudaStream_t stream) {
   if (!gemm_f32_split_scratch_bytes(m, n, k, ldc) || !scratch)
     return "the shape is not for the tensor-core f32 product";
-  int *row_flags = (int *)scratch, *column_flags = row_flags + (m + TILE - 1) / TILE;
-  __nv_bfloat16 *a6 = (__nv_bfloat16 *)((char *)scratch + flag_bytes(m, n));
+  const Flags f = flags_of(scratch, m, n, k);
+  __nv_bfloat16 *a6 = (__nv_bfloat16 *)((char *)scratch + flag_bytes(m, n, k));
   __nv_bfloat16 *b6 = a6 + m * 6 * k;
   float *partials = (float *)((char *)a6 + up256((size_t)(m + n) * 6 * k * 2));
   const uint32_t limit = too_large(k);
-  if (cudaMemsetAsync(row_flags, 0, flag_bytes(m, n), stream) != cudaSuccess)
-    return "the flags of the f32 product could not be cleared";
-  launch_chained(split_a_kernel, dim3((unsigned)((m * (k / 8) + 255) / 256)), dim3(256),
-                 0, stream, a6, a, lda, (int)m, (int)k, limit, row_flags);
-  launch_chained(split_bt_kernel, dim3((unsigned)((n + 31) / 32), (unsigned)((k + 31) / 32)),
-                 dim3(256), 0, stream, b6, b, ldb, (int)k, (int)n, limit, column_flags);
+  launch_chained(split_bt_kernel, dim3((unsigned)f.across, (unsigned)f.down), dim3(256), 0,
+                 stream, b6, b, ldb, (int)k, (int)n, limit, f);
+  launch_chained(split_a_kernel,
+                 dim3((unsigned)((m * (k / 8) + 255) / 256 + (n + TILE - 1) / TILE)),
+                 dim3(256), 0, stream, a6, a, lda, (int)m, (int)k, limit, f);
   if (cudaGetLastError() != cudaSuccess)
     return "the term-splitting launches failed";
   int splits = runs_of(m, n, k);
@@ -274,7 +315,7 @@ const char *gemm_f32_split(const float *a, int64_t lda, const float *b, int64_t 
   launch_chained(plain_tiles_kernel, dim3((unsigned)std::min<int64_t>(tiles, sm_count())),
                  dim3(kPlainThreads), room, stream,
                  PlainTile{a, b, lda, ldb, (int)m, (int)n, vec(a, lda), vec(b, ldb)}, c, ldc,
-                 (int)k, (const int *)row_flags, (const int *)column_flags);
+                 (int)k, (const int *)f.rows, (const int *)f.columns);
   if (cudaGetLastError() != cudaSuccess)
     return "the launch of the plain tiles failed";
   return nullptr;

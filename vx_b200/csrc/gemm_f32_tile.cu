@@ -384,17 +384,18 @@ int blocks_of_tile(int64_t m, int64_t n, int64_t k) {
 
 } // namespace
 
-/* Microseconds, about: 1.9 for a block of K of a tile (3 700 cycles: 96 KiB of terms
-   written to shared memory and 176 KiB read from it, and sixteen warps splitting),
-   as many rounds as the tiles need. Measured 24.8 / 51.4 / 126 / 365 at 1024^3, 1536^3,
-   2048^3, 3072^3, where this gives 21 / 52 / 128 / 371. */
+/* Microseconds, about: 1.7 for a block of K of a tile (96 KiB of terms written to shared
+   memory and 176 KiB read from it, and sixteen warps splitting) and 7.4 for a tile's start
+   and end, as many rounds as the tiles need. Measured 24.6 / 51.4 / 126 / 365 / 65.6 / 38.8
+   at 1024^3, 1536^3, 2048^3, 3072^3, 2944 x 2944 x 320, 128 x 128 x 8192, where this gives
+   24.6 / 51.8 / 127 / 360 / 67 / 38.2. */
 double gemm_f32_tile_us(int64_t m, int64_t n, int64_t k) {
   if ((m + BM - 1) / BM > kMostRowTiles)
     return HUGE_VAL;
   const int64_t z = blocks_of_tile(m, n, k);
   const int64_t blocks = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * z;
   const int64_t k_blocks = ((k + BK - 1) / BK + z - 1) / z;
-  return 6.0 + 1.9 * (double)((blocks + sm_count() - 1) / sm_count() * k_blocks);
+  return 3.6 + (double)((blocks + sm_count() - 1) / sm_count()) * (7.4 + 1.7 * k_blocks);
 }
 
 const char *gemm_f32_tile(const float *a, int64_t lda, const float *b, int64_t ldb,
