@@ -498,7 +498,11 @@ int32_t vx_b200_flash_attention(const void *q, const void *k, const void *v,
    The arithmetic of nn_moe_swiglu_q4_rows / nn_moe_down_q4_add_rows
    (nn.vx:2958, 3066) in another order of sums: results agree with the
    vx_nn_*_rows exports within rounding, not bit for bit. rows a multiple of 8,
-   cols of 32 (fastest with cols a multiple of 128). */
+   cols of 32 (fastest with cols a multiple of 128). Experts of 32 pairs or more
+   take up to 1 GiB of device memory for the call, in the order of the caller's
+   stream; what is freed is kept within VX_CUDA_POOL_MAX_MB, and without it the
+   call runs as for fewer pairs. Scales are finite: one of infinity makes results
+   NaN or infinite, which of the two depends on the number of pairs. */
 /* y[n, rows] = x[n, cols] . W^T for a Q4_0 matrix W [rows, cols] (codes 8 to a
    u32 word, an f16 scale per 32 weights of a row: the layout of nn_matvec_q4,
    nn.vx:1645-1666) and n rows of f32 activations, on the tensor cores: the

@@ -2,8 +2,10 @@
  * f32 cache, on the tensor cores (nn_attention, nn.vx:349-866, for every position).
  *
  * A block per (128 positions, query head), head_dim 128; 64 keys at a time.  An f32
- * value is the exact sum of three bf16 terms, and a product keeps the six largest of
- * the nine term products (what is dropped is below 2^-24 of it), as in gemm_f32_tile.cu:
+ * value from 2^-109 on is the exact sum of three bf16 terms (below, the third is cut to
+ * the subnormals: 2^-134 of one is lost, as in the output's own terms), and a product
+ * keeps the six largest of the nine term products (what is dropped is below 2^-24 of it),
+ * as in gemm_f32_tile.cu:
  *
  *   scores   q1 [k1 | k2 | k3], q2 [k1 | k2], q3 k1: the terms of a tile of keys lie
  *            one after another along N, so three instructions a K step do all six
@@ -30,7 +32,8 @@
  *
  * Magnitudes from 2^56 on, infinities and NaN, whose terms or products could overflow
  * where the scores do not, are noticed while they are read; a block that met one
- * computes its rows with plain multiply-adds instead.
+ * computes its rows with plain multiply-adds as well, a key after another: 1.2 ms for
+ * one head of 32 over 500 positions.
  */
 #include "kernels.h"
 #include "launch.cuh"

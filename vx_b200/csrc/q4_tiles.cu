@@ -7,10 +7,11 @@
  * significant bits: two bf16 terms hold it exactly, and they are made on the way into
  * tensor memory, the A operand; x is three bf16 terms in shared memory.  Of the six
  * products the smallest (below 2^-24 of the first) is left out.  The tensor core's own
- * sums lose a little with their length: the first product has an accumulator of its own, which is added to f32 registers after 128 columns, while the
- * other products of the next block run (with 512 columns the layer's error against 64 bits
- * was 9.1e-7, on mma.sync with a sum per 32 columns 5.9e-7); the others, 2^-8 of it, stay
- * in theirs to the end.
+ * sums lose a little with their length: the first product has an accumulator of its own,
+ * which is added to f32 registers after 128 columns, while the other products of the next
+ * block run (the layer's error against 64 bits is 3.5e-7; with 512 columns it was 9.1e-7, on
+ * mma.sync with a sum per 32 columns 5.9e-7); the others, 2^-8 of it, stay in theirs to the
+ * end.
  *
  * Sixteen warps, persistent over (segment of pairs, row tile), with rings of three blocks
  * of 64 columns:
@@ -27,6 +28,9 @@
  * 2 000 cycles a block of 64 columns) and the round of barriers between it and the sets for
  * the rest; with few pairs that round alone, 1 250 cycles.  The gate and up rows of 8
  * experts of 14336 x 4096 take 0.93 ms for 1000 pairs, 2.5 ms on mma.sync (moe_grouped.cu).
+ *
+ * A scale of infinity makes its 32 weights NaN (its second term is infinity minus
+ * infinity); moe_grouped.cu, which applies the scale to the sum of the 32, gives infinity.
  *
  * What was slower: the codes alone as A (exact, three products) and the scale applied to
  * the sums of each 32 columns, 1 850 cycles a block of few pairs and 2 500 of 128, since
