@@ -99,8 +99,8 @@ def test_f32_ragged_shapes(oracle, m, n, k):
 @pytest.mark.parametrize("m,n,k", [(1024, 1024, 1024), (300, 260, 128),
                                    (257, 512, 192), (128, 4096, 64)])
 def test_f32_on_the_tensor_cores_is_as_good_as_the_fp32_kernel(m, n, k, monkeypatch):
-    """An f32 product large enough runs as exact bf16 terms on the tensor
-    cores (k a multiple of 64, n of 4). Against an f64 product its error must
+    """An f32 product runs as exact bf16 terms on the tensor cores, made inside the
+    kernel at these sizes. Against an f64 product its error must
     be of the size of the FP32 kernel's own, and both far inside the 1e-4 of
     the reference's check."""
     rng = np.random.default_rng(m + n + k)
@@ -146,9 +146,8 @@ def test_strided_view_with_offset(oracle):
 
 
 def test_strided_views_on_the_tensor_core_f32_route():
-    """Views large enough for the tensor-core route: A and B inside wider
-    buffers at an offset, C into the middle of a wider buffer (row stride >
-    width, so the partial sums go through the adding kernel)."""
+    """A and B inside wider buffers at an offset, C into the middle of a wider
+    buffer (the same for terms made beforehand: test_gpu_matmul_any_shape.py)."""
     rng = np.random.default_rng(19)
     abig = rng.uniform(-1, 1, (300, 200)).astype(np.float32)
     bbig = rng.uniform(-1, 1, (140, 520)).astype(np.float32)

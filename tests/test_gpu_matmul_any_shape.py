@@ -247,3 +247,25 @@ def test_f32_products_of_more_rows_than_tiles_in_a_grid():
         want = a[at:at + 300].double() @ b.double()
         assert ((c[at:at + 300] - want).norm() / want.norm()).item() <= 1e-6
     assert ops.kernel_status() == 0
+
+
+def test_f32_products_of_a_long_k():
+    """Values of one sign over 26624 of K, terms made beforehand: runs of at most 12288,
+    whose sums are cut at each step of 16 by at most 2^-24, where one run would be 7.6e-5
+    off."""
+    import torch
+    m, n, k = 2304, 2048, 26624
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    a = torch.rand((m, k), generator=g, device="cuda")
+    b = torch.rand((k, n), generator=g, device="cuda")
+    c = torch.zeros((m, n), device="cuda")
+    t = [abi.DeviceTensor(x.data_ptr(), tuple(x.shape), abi.F32, abi.home_gpu())
+         for x in (c, a, b)]
+    torch.cuda.synchronize()
+    ops.matmul_into(*t)
+    torch.cuda.synchronize()
+    for at in (0, 1000, m - 64):
+        want = a[at:at + 64].double() @ b.double()
+        assert ((c[at:at + 64] - want).norm() / want.norm()).item() <= 12288 / 16 * 2.0 ** -24
+    assert ops.kernel_status() == 0

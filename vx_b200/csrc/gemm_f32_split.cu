@@ -10,7 +10,7 @@
  * as ONE bf16 GEMM over K' = 6 k:
  *   A' [m, 6k] = a3 | a2 | a1 | a2 | a1 | a1
  *   B' [n, 6k] = b1 | b2 | b3 | b1 | b2 | b1      (B transposed on the way)
- * -- the small products first: the tensor core cuts its sum off at every K step of 16, by
+ * (of each run of K by itself, one run after another) -- the small products first: the tensor core cuts its sum off at every K step of 16, by
  * up to 2^-24 of what the sum then is, so only the k / 16 steps of a1 b1 count.  With a1 b1
  * first 3072^3 in one run was 3.4e-5 off (2.0e-5 of values in [0, 1)), so it is 2.9e-6
  * (8.9e-6).  It runs on the CTA-pair kernel of the prefill (tcgen05.mma.cta_group::2,
@@ -63,12 +63,32 @@ __device__ __forceinline__ void three_terms(float v, __nv_bfloat16 &t1,
   t3 = __float2bfloat16(r1 - __bfloat162float(t2));
 }
 
+/* Where the terms of a block of 64 of K lie: the first is block `first` of K', the next one
+   is `step` further. Run r of `runs` has the blocks r * blocks / runs .. of K. */
+struct Place {
+  int64_t first;
+  int step;
+};
+template <typename Int> __device__ __forceinline__ Place place_in(int block, int blocks, int runs) {
+  const int r = (int)(((Int)(block + 1) * runs - 1) / blocks);
+  const int begin = (int)((Int)r * blocks / runs);
+  const int end = (int)((Int)(r + 1) * blocks / runs);
+  return Place{6 * (int64_t)begin + (block - begin), end - begin};
+}
+__device__ __forceinline__ Place place_of(int block, int blocks, int runs) {
+  if (runs == 1)
+    return Place{block, blocks};
+  /* three 64-bit divisions cost a thread as much as the rest of its work */
+  return (uint64_t)(blocks + 1) * runs < (1ull << 32) ? place_in<uint32_t>(block, blocks, runs)
+                                                     : place_in<uint64_t>(block, blocks, runs);
+}
+
 /* A' from A: one thread per eight consecutive values of a row (k is a
    multiple of 64), six 16-byte stores. The last blocks gather the flags that split_bt's
    blocks left, one block for each 128 columns. */
 __global__ void __launch_bounds__(256)
 split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k,
-               uint32_t limit, const Flags f) {
+               int runs, uint32_t limit, const Flags f) {
   chain_release();
   chain_wait();
   const int gatherers = (f.across + 3) / 4;
@@ -107,20 +127,22 @@ split_a_kernel(__nv_bfloat16 *out, const float *a, int64_t lda, int m, int k,
   const uint4 t3 = make_uint4(w3[0], w3[1], w3[2], w3[3]);
   if (most >= limit)
     f.rows[r / TILE] = 1;
-  __nv_bfloat16 *row = out + r * 6 * k + c;
+  const Place at = place_of(c / 64, k / 64, runs);
+  const int64_t step = (int64_t)at.step * 64;
+  __nv_bfloat16 *row = out + r * 6 * k + at.first * 64 + c % 64;
   *reinterpret_cast<uint4 *>(row) = t3;
-  *reinterpret_cast<uint4 *>(row + k) = t2;
-  *reinterpret_cast<uint4 *>(row + 2 * (int64_t)k) = t1;
-  *reinterpret_cast<uint4 *>(row + 3 * (int64_t)k) = t2;
-  *reinterpret_cast<uint4 *>(row + 4 * (int64_t)k) = t1;
-  *reinterpret_cast<uint4 *>(row + 5 * (int64_t)k) = t1;
+  *reinterpret_cast<uint4 *>(row + step) = t2;
+  *reinterpret_cast<uint4 *>(row + 2 * step) = t1;
+  *reinterpret_cast<uint4 *>(row + 3 * step) = t2;
+  *reinterpret_cast<uint4 *>(row + 4 * step) = t1;
+  *reinterpret_cast<uint4 *>(row + 5 * step) = t1;
 }
 
 /* B' from B [k, n]: a block transposes a 32 x 32 tile through shared memory,
    so that B is read along n and B' written along k. */
 __global__ void __launch_bounds__(256)
 split_bt_kernel(__nv_bfloat16 *out, const float *b, int64_t ldb, int k, int n,
-                uint32_t limit, const Flags f) {
+                int runs, uint32_t limit, const Flags f) {
   __shared__ __nv_bfloat16 tile[3][32][34];
   chain_release();
   chain_wait();
@@ -143,17 +165,19 @@ split_bt_kernel(__nv_bfloat16 *out, const float *b, int64_t ldb, int k, int n,
   for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
        i < f.row_tiles; i += (int64_t)gridDim.x * gridDim.y * blockDim.x)
     f.rows[i] = 0;
+  const Place at = place_of(k0 / 64, k / 64, runs); /* 32 of K are of one block */
+  const int64_t step = (int64_t)at.step * 64;
   for (int j = ty; j < 32; j += 8) {
     if (n0 + j >= n || k0 + tx >= k)
       continue;
-    __nv_bfloat16 *row = out + (int64_t)(n0 + j) * 6 * k + k0 + tx;
+    __nv_bfloat16 *row = out + (int64_t)(n0 + j) * 6 * k + at.first * 64 + k0 % 64 + tx;
     const __nv_bfloat16 t1 = tile[0][tx][j], t2 = tile[1][tx][j], t3 = tile[2][tx][j];
     row[0] = t1;
-    row[k] = t2;
-    row[2 * (int64_t)k] = t3;
-    row[3 * (int64_t)k] = t1;
-    row[4 * (int64_t)k] = t2;
-    row[5 * (int64_t)k] = t1;
+    row[step] = t2;
+    row[2 * step] = t3;
+    row[3 * step] = t1;
+    row[4 * step] = t2;
+    row[5 * step] = t1;
   }
 }
 
@@ -229,14 +253,16 @@ bool direct(int splits, int64_t n, int64_t ldc) { return splits == 1 && ldc == n
 
 /* How many runs the K blocks are cut into: the number, up to 12, that leaves the
    last wave of pairs fullest. Many short runs rather than the fewest that are as
-   fast: the tensor core's own f32 sums lose a little with their length (1024^3 with
-   a1 b1 first in 4 runs: relative error 2.2e-6, in 9: 9e-7). */
+   fast: the tensor core's own f32 sums lose a little with their length, and none is
+   longer than 12288 of K: 768 cuts of up to 2^-24 are 4.6e-5, where the reference's
+   check of a product allows 1e-4. */
 int runs_of(int64_t m, int64_t n, int64_t k) {
   const int tiles = (int)(((m + 255) / 256) * ((n + 255) / 256));
-  const int k_blocks = (int)(6 * k / 64), pairs = 74;
-  int best = 1;
+  const int blocks = (int)(k / 64), pairs = 74;
+  const int least = (int)((k + 12287) / 12288);
+  int best = least;
   double best_fill = 0.0;
-  for (int s = 1; s <= 12 && s <= k_blocks; ++s) {
+  for (int s = least; s <= std::max(12, least) && s <= blocks; ++s) {
     const int items = tiles * s;
     const double fill = (double)items / (((items + pairs - 1) / pairs) * pairs);
     if (fill > best_fill + 0.02) {
@@ -285,17 +311,17 @@ const char *gemm_f32_split(const float *a, int64_t lda, const float *b, int64_t 
   __nv_bfloat16 *b6 = a6 + m * 6 * k;
   float *partials = (float *)((char *)a6 + up256((size_t)(m + n) * 6 * k * 2));
   const uint32_t limit = too_large(k);
+  int splits = runs_of(m, n, k);
   launch_chained(split_bt_kernel, dim3((unsigned)f.across, (unsigned)f.down), dim3(256), 0,
-                 stream, b6, b, ldb, (int)k, (int)n, limit, f);
+                 stream, b6, b, ldb, (int)k, (int)n, splits, limit, f);
   launch_chained(split_a_kernel,
                  dim3((unsigned)((m * (k / 8) + 255) / 256 + (n + TILE - 1) / TILE)),
-                 dim3(256), 0, stream, a6, a, lda, (int)m, (int)k, limit, f);
+                 dim3(256), 0, stream, a6, a, lda, (int)m, (int)k, splits, limit, f);
   if (cudaGetLastError() != cudaSuccess)
     return "the term-splitting launches failed";
-  int splits = runs_of(m, n, k);
   float *out = direct(splits, n, ldc) ? c : partials;
   if (const char *why = rows_gemm_of(a6, 6 * k, b6, 6 * k, (int)m, (int)n, out, &splits,
-                                     stream, splits, kDown))
+                                     stream, splits, kDown, 6))
     return why;
   if (out != c) {
     const int vec = ldc % 4 == 0 && ((uintptr_t)c & 15) == 0;

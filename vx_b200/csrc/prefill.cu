@@ -71,6 +71,7 @@ struct RowsGemm {
   int splits;
   float *partials; /* [splits][t][n] */
   float scale;     /* of the sums */
+  int unit;        /* K' blocks that stay in one run; k_blocks is a multiple */
 };
 
 /* Item -> (tile of positions, tile of weight rows, run). The runs and position
@@ -124,7 +125,9 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap map_x,
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
   /* the K' blocks of run r: a balanced cut of 0 .. k_blocks */
-  auto run_first = [&](int r) { return (int)((int64_t)r * g.k_blocks / g.splits); };
+  auto run_first = [&](int r) {
+    return (int)((int64_t)r * (g.k_blocks / g.unit) / g.splits) * g.unit;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -605,7 +608,8 @@ const char *rows_gemm(const void *terms, const void *w, int t, int n, int cols,
 
 const char *rows_gemm_of(const void *terms, int64_t term_cols, const void *w,
                          int64_t w_cols, int t, int n, float *partials,
-                         int *splits_out, cudaStream_t stream, int splits, float scale) {
+                         int *splits_out, cudaStream_t stream, int splits, float scale,
+                         int unit) {
   if (term_cols % BK != 0 || w_cols % BK != 0)
     return "the multi-position projections need columns in multiples of 64";
   if (allow_dynamic_smem((const void *)rows_gemm_kernel, SMEM_BYTES) != cudaSuccess)
@@ -623,6 +627,7 @@ const char *rows_gemm_of(const void *terms, int64_t term_cols, const void *w,
   g.splits = splits > 0 ? splits : rows_gemm_splits_of(t, n, term_cols);
   g.partials = partials;
   g.scale = scale;
+  g.unit = unit;
   *splits_out = g.splits;
   int pairs = resident_pairs();
   if (pairs < 1)
