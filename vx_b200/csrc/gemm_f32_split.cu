@@ -19,8 +19,8 @@
  * The range is that of gemm_f32_tile.cu: both operands times 2^24, the sums times 2^-48,
  * and a flag for each 128 rows of A and 128 columns of B in which a value was met that is
  * too large then (infinities and NaN among them).  A last launch computes the tiles of
- * flagged rows and columns with plain multiply-adds; where there is none it adds 1.3 us
- * to the 289 of 3072^3.
+ * flagged rows and columns with plain multiply-adds; where there is none it adds 1.4
+ * to 3 us (3072 x 3072 x 1024: 103.7 -> 105.1, 3072 x 3072 x 64: 30.0 -> 33.0).
  */
 #include "kernels.h"
 #include "launch.cuh"
