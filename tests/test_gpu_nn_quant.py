@@ -88,6 +88,47 @@ def test_swiglu(oracle, quant, rows, cols):
     close(tout.to_host(), oracle.quant_swiglu(quant, w, s, x, rows, cols), 4e-6)
 
 
+@pytest.mark.parametrize("rows,cols", [
+    (4, 256),           # fewer pairs of rows than SMs, one step a row
+    (2372, 512),        # a tile of eight pairs and two more on an SM
+    (44000, 256),       # more tiles an SM than the warps meet for at once
+    (300, 11008),       # steps that do not divide by the warps
+    (64, 18432),        # one block an SM
+    (16, 39936), (16, 40960)])  # the longest rows, and too long for shared memory
+@pytest.mark.parametrize("values", ["normal", "apart", "small", "large"])
+def test_q4_rows(oracle, rows, cols, values):
+    """Every row within the f32 roundings of its sum: one for each 32 columns, and twenty
+    more where the parts of a sum meet, each at most 2^-24 of the sum of magnitudes; x
+    itself is off by at most 2^-38 of the largest of its 32, weights by none."""
+    w, s = oracle.quant_inputs("q4", rows, cols, 5)
+    x = oracle.random_f32(cols, 6, 1.0)
+    if values == "apart":           # one of 64 far above the others
+        x[::64] *= np.float32(1e5)
+    x *= {"small": np.float32(1e-33), "large": np.float32(1e30)}.get(values, np.float32(1))
+    ty = abi.DeviceTensor.empty((rows,), abi.F32)
+    ops.nn_matvec_quant("q4", ty, dev(w), dev(s), dev(x), rows, cols)
+    codes = (w.view(np.uint32).reshape(rows, -1, 1) >> np.arange(0, 32, 4, dtype=np.uint32)) & 15
+    scales = np.repeat(s.view(np.float16).reshape(rows, -1).astype(np.float64), 32, axis=1)
+    weights = (codes.reshape(rows, cols).astype(np.float64) - 8.0) * scales
+    top = np.repeat(np.abs(x.reshape(-1, 32)).max(1), 32).astype(np.float64)
+    size = np.abs(weights) @ np.abs(x.astype(np.float64))
+    bound = (cols / 32 + 20) * 2.0 ** -24 * size + np.abs(weights) @ top * 2.0 ** -38
+    off = np.abs(ty.to_host().astype(np.float64) - weights @ x.astype(np.float64))
+    assert (off <= bound + 1e-45).all(), (off / np.maximum(bound, 1e-300)).max()
+
+
+def test_q4_not_a_number(oracle):
+    """An infinity or a NaN in x makes every row NaN."""
+    rows, cols = 8, 512
+    w, s = oracle.quant_inputs("q4", rows, cols, 5)
+    for bad in (np.inf, np.nan):
+        x = oracle.random_f32(cols, 6, 1.0)
+        x[77] = bad
+        ty = abi.DeviceTensor.empty((rows,), abi.F32)
+        ops.nn_matvec_quant("q4", ty, dev(w), dev(s), dev(x), rows, cols)
+        assert np.isnan(ty.to_host()).all()
+
+
 def test_every_fp8_code(oracle):
     """Each non-NaN code alone in a row with scale 1 and x = 1: the hardware
     conversion must give the value of the f8e4m3 definition, bit for bit."""

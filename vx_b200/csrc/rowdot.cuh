@@ -17,6 +17,7 @@
 #include <cuda_fp16.h>
 
 #include <cstdio>
+#include <climits>
 #include <cstdlib>
 
 namespace vxb {

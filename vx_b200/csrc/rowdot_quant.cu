@@ -1,16 +1,18 @@
 /* rowdot_quant.cu -- the projections with fp8 and Q4_0 weights: on the tensor
- * cores where the shape allows (rowdot_quant_mma.cuh), else on the FMA pipe. */
+ * cores where the shape allows (rowdot_quant_mma.cuh: fp8, rowdot_q4_int.cuh: Q4_0), else
+ * on the FMA pipe. */
 #include "rowdot.cuh"
 
 namespace vxb {
 namespace {
 
 #include "rowdot_quant_mma.cuh"
+#include "rowdot_q4_int.cuh"
 
 template <int EPI>
 const char *either_format(RowDotParams &p, int fmt, cudaStream_t stream) {
-  const char *r = fmt == kFmtFp8 ? launch_quant_mma<Fp8W, EPI>(p, stream)
-                                 : launch_quant_mma<Q4W, EPI>(p, stream);
+  const char *r = fmt == kFmtFp8 ? launch_quant_mma<EPI>(p, stream)
+                                 : launch_q4_int<EPI>(p, stream);
   if (!r || r[0])
     return r;
   return fmt == kFmtFp8 ? launch_rowdot_b<Fp8W, 1, EPI>(p, stream)

@@ -1,17 +1,15 @@
-/* rowdot_quant_mma.cuh -- the fp8 and Q4_0 projections of ONE sequence on the
- * tensor cores (nn_matvec_fp8 / nn_swiglu_fp8 / nn_qkv_fp8, nn.vx:1306-1577;
- * the Q4_0 forms, nn.vx:1666-2190). Part of rowdot_quant.cu (included there).
+/* rowdot_quant_mma.cuh -- the fp8 projections of ONE sequence on the tensor cores
+ * (nn_matvec_fp8 / nn_swiglu_fp8 / nn_qkv_fp8, nn.vx:1306-1577), and the epilogues that
+ * rowdot_q4_int.cuh shares. Part of rowdot_quant.cu (included there).
  *
- * With one-byte and half-byte weights the projection kernel is bound by
- * instruction issue, not by HBM: every weight costs a conversion to f32, a
- * multiply-add and its share of the loads (six instructions per weight and
- * lane).  Here a warp takes 16 weight rows at a time as the A operand of
- * mma.sync.m16n8k16, and the f32 activations enter as the B operand split into
- * three 16-bit terms whose sum is x exactly (bf16 terms beside Q4_0 codes,
- * which become small bf16 integers; f16 terms, the second and third scaled by
- * 2^11 and 2^22, beside fp8 codes, which the conversion instruction turns into
- * f16 two at a time).  The products are exact in f32 and the tensor core
- * accumulates them in f32, so a weight costs a fraction of an instruction.
+ * With one-byte weights the projection kernel is bound by instruction issue, not by HBM:
+ * every weight costs a conversion to f32, a multiply-add and its share of the loads (six
+ * instructions per weight and lane).  Here a warp takes 16 weight rows at a time as the A
+ * operand of mma.sync.m16n8k16, and the f32 activations enter as the B operand split into
+ * three f16 terms whose sum is x exactly, the second and third scaled by 2^11 and 2^22
+ * (the conversion instruction turns fp8 codes into f16 two at a time).  The products are
+ * exact in f32 and the tensor core accumulates them in f32, so a weight costs a fraction
+ * of an instruction.
  *
  * The 16 rows of a warp's tile are the two rows of eight ITEMS of the
  * projection kernel (rows g and g + 8 of the A operand are rows r0 and r1 of
@@ -21,10 +19,9 @@
  * lane reads its codes and its activations with wide loads.
  *
  * Weights arrive through a per-warp ring filled by TMA: two tiled copies per
- * k-step, each eight rows of 128 bytes (the eight r0 rows, the eight r1 rows;
- * for Q4_0 two more bring the rows' f16 scales of the step), 128-byte swizzled
- * so that the lanes' loads do not meet in a bank.  (One bulk copy per row was
- * correct and slower than the FMA-pipe kernel: 700 000 copies of 128 bytes per
+ * k-step, each eight rows of 128 bytes (the eight r0 rows, the eight r1 rows),
+ * 128-byte swizzled so that the lanes' loads do not meet in a bank.  (One bulk copy per
+ * row was correct and slower than the FMA-pipe kernel: 700 000 copies of 128 bytes per
  * projection kept the copy unit, not HBM, busy.)  With fewer tiles
  * than warps the k-steps of a tile are divided among 2, 4, 8 or 16
  * neighbouring warps, whose partial sums meet in shared memory in a fixed
@@ -38,17 +35,8 @@ constexpr int STEP_ROW_BYTES = 128; /* of one row per k-step */
 
 __device__ int g_quant_status; /* non-zero: a ring wait gave up */
 
-template <typename W> struct QFmt;
-template <> struct QFmt<Fp8W> {
-  static constexpr int codes = 128;       /* per row and k-step: one block of scales */
-  static constexpr int scale_bytes = 0;   /* scales are read from global memory */
-  static constexpr int x_pad = 16;        /* bytes between the terms' rows, mod 128 */
-};
-template <> struct QFmt<Q4W> {
-  static constexpr int codes = 256;
-  static constexpr int scale_bytes = 256; /* 16 rows x eight f16 per k-step */
-  static constexpr int x_pad = 64;
-};
+constexpr int STEP_COLS = 128; /* of a row per k-step: one block of scales */
+constexpr int X_PAD = 16;      /* bytes between the terms' rows, mod 128 */
 constexpr int STAGE_CODES_BYTES = 2048; /* two boxes of 8 rows x 128 bytes */
 constexpr int MAX_STAGES = 8;
 
@@ -97,13 +85,6 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4],
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4],
-                                         uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
-               "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 /* the two fp8 (e4m3) codes in the low (HI = false) or high 16 bits of `four`,
    as two f16: the lower byte in the lower half */
 template <bool HI> __device__ __forceinline__ uint32_t fp8x2_to_f16x2(uint32_t four) {
@@ -120,25 +101,38 @@ template <bool HI> __device__ __forceinline__ uint32_t fp8x2_to_f16x2(uint32_t f
         : "r"(four));
   return out;
 }
-__device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
+/* What the epilogue of an item reads from the kernels before: the two values that its
+   results are added to, or the cosine and sine of its pair. */
+template <int EPI>
+__device__ __forceinline__ float2 before_item(const RowDotParams &p, int item) {
+  float2 v = make_float2(0.0f, 0.0f);
+  if (EPI == EPI_ADD) {
+    v.x = p.y[2 * item];
+    if (2 * item + 1 < p.rows)
+      v.y = p.y[2 * item + 1];
+  } else if (EPI == EPI_QKV) {
+    const int half = p.head_dim / 2;
+    const int head = item / half;
+    if (head < p.q_heads + p.kv_heads) {
+      const int64_t at = (int64_t)p.positions[0] * p.cs_cols + item - head * half;
+      v = make_float2(p.cos_t[at], p.sin_t[at]);
+    }
+  }
+  return v;
 }
 
 /* What lane 0 of the projection kernel does with the two results of an item,
    for one sequence (the epilogues of rowdot_kernel). */
 template <int EPI>
-__device__ __forceinline__ void finish_item(const RowDotParams &p, int item, float t0,
-                                            float t1) {
+__device__ __forceinline__ void finish_item_with(const RowDotParams &p, int item, float t0,
+                                                 float t1, float2 read) {
   if (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_BIAS) {
     const int ra = 2 * item, rb = 2 * item + 1;
     const bool two = rb < p.rows;
     float v0 = t0, v1 = t1;
     if (EPI == EPI_ADD) {
-      v0 = p.y[ra] + v0;
-      if (two)
-        v1 = p.y[rb] + v1;
+      v0 = read.x + v0;
+      v1 = read.y + v1;
     } else if (EPI == EPI_BIAS) {
       v0 += bf16_at(p.bias, ra);
       if (two)
@@ -167,8 +161,7 @@ __device__ __forceinline__ void finish_item(const RowDotParams &p, int item, flo
       vrow[ib] = vb;
       return;
     }
-    const float c = p.cos_t[(int64_t)pos * p.cs_cols + idx];
-    const float s = p.sin_t[(int64_t)pos * p.cs_cols + idx];
+    const float c = read.x, s = read.y;
     const float oa = __fsub_rn(__fmul_rn(va, c), __fmul_rn(vb, s));
     const float ob = __fadd_rn(__fmul_rn(vb, c), __fmul_rn(va, s));
     float *dst = head < p.q_heads
@@ -177,6 +170,11 @@ __device__ __forceinline__ void finish_item(const RowDotParams &p, int item, flo
     dst[ia] = oa;
     dst[ib] = ob;
   }
+}
+template <int EPI>
+__device__ __forceinline__ void finish_item(const RowDotParams &p, int item, float t0,
+                                            float t1) {
+  finish_item_with<EPI>(p, item, t0, t1, before_item<EPI>(p, item));
 }
 
 struct QuantPlan {
@@ -189,24 +187,18 @@ struct QuantPlan {
   int warps, stages;
 };
 
-template <typename W, int EPI>
+template <int EPI>
 __global__ void __launch_bounds__(QTHREADS, 1)
 quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
                  const __grid_constant__ CUtensorMap map_a,
-                 const __grid_constant__ CUtensorMap map_b,
-                 const __grid_constant__ CUtensorMap map_sa,
-                 const __grid_constant__ CUtensorMap map_sb) {
-  typedef QFmt<W> F;
-  constexpr bool FP8 = F::codes == 128;
+                 const __grid_constant__ CUtensorMap map_b) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   /* swizzled boxes want 1 KiB alignment */
   unsigned char *smem_dyn =
       smem_raw + ((1024 - (ptx::smem_addr(smem_raw) & 1023)) & 1023);
   const int stages = plan.stages, nwarps = plan.warps;
   const int nthreads = nwarps * 32;
-  /* a warp's ring: its stages of codes, then its stages of scales, rounded up
-     to the 1 KiB the swizzled boxes of the next warp want */
-  const int warp_ring = (stages * (STAGE_CODES_BYTES + F::scale_bytes) + 1023) & ~1023;
+  const int warp_ring = stages * STAGE_CODES_BYTES;
   unsigned char *ring = smem_dyn;
   unsigned char *xterms = smem_dyn + nwarps * warp_ring;
   __shared__ float ssq[WARPS];
@@ -216,9 +208,8 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int cols = p.cols;
-  const int xstride = x_term_stride(cols, F::x_pad);
+  const int xstride = x_term_stride(cols, X_PAD);
   unsigned char *my_ring = ring + warp * warp_ring;
-  unsigned char *my_scales = my_ring + stages * STAGE_CODES_BYTES;
 
   if (lane == 0) {
     for (int s = 0; s < stages; ++s)
@@ -234,7 +225,7 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
   const int rounds = (int)((units + total_warps - 1) / total_warps);
 
   /* ---- the loading side: one unit (a tile's share of the k-steps) at a time;
-     lane 0 issues two (Q4_0: four) tiled copies per k-step. ya, yb: the rows
+     lane 0 issues two tiled copies per k-step. ya, yb: the rows
      of the two maps where the tile's r0 and r1 rows begin. ---- */
   int ld_stage = 0, ld_ks = 0, ld_end = 0, issued = 0, ld_ya = 0, ld_yb = 0;
   auto open_unit = [&](int64_t u) {
@@ -256,14 +247,9 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
     if (lane == 0) {
       unsigned char *dst = my_ring + ld_stage * STAGE_CODES_BYTES;
       uint64_t *bar = &bars[warp][ld_stage];
-      ptx::mbar_expect_tx(bar, STAGE_CODES_BYTES + F::scale_bytes);
+      ptx::mbar_expect_tx(bar, STAGE_CODES_BYTES);
       ptx::tma_load_2d(dst, &map_a, ld_ks * STEP_ROW_BYTES, ld_ya, bar);
       ptx::tma_load_2d(dst + 1024, &map_b, ld_ks * STEP_ROW_BYTES, ld_yb, bar);
-      if (!FP8) {
-        unsigned char *sd = my_scales + ld_stage * F::scale_bytes;
-        ptx::tma_load_2d(sd, &map_sa, ld_ks * 16, ld_ya, bar);
-        ptx::tma_load_2d(sd + 128, &map_sb, ld_ks * 16, ld_yb, bar);
-      }
     }
     ++issued;
     ++ld_ks;
@@ -303,30 +289,16 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
       for (int j = 0; j < 4; ++j) {
         const int i = 4 * q + j;
         unsigned short t1, t2, t3;
-        int at = i;
-        if (FP8) {
-          const __half h1 = __float2half_rn(e[j]);
-          const float r1 = (e[j] - __half2float(h1)) * 2048.0f;
-          const __half h2 = __float2half_rn(r1);
-          const float r2 = (r1 - __half2float(h2)) * 2048.0f;
-          t1 = __half_as_ushort(h1);
-          t2 = __half_as_ushort(h2);
-          t3 = __half_as_ushort(__float2half_rn(r2));
-        } else {
-          const __nv_bfloat16 b1 = __float2bfloat16_rn(e[j]);
-          const float r1 = e[j] - __bfloat162float(b1);
-          const __nv_bfloat16 b2 = __float2bfloat16_rn(r1);
-          const float r2 = r1 - __bfloat162float(b2);
-          t1 = __bfloat16_as_ushort(b1);
-          t2 = __bfloat16_as_ushort(b2);
-          t3 = __bfloat16_as_ushort(__float2bfloat16_rn(r2));
-          /* inside a run of 8 the order is 0 4 1 5 2 6 3 7: the codes of a
-             32-bit word pair up as (0, 4), (1, 5), (2, 6), (3, 7) */
-          at = (i & ~7) | ((i & 3) * 2 + ((i >> 2) & 1));
-        }
-        *reinterpret_cast<unsigned short *>(xterms + at * 2) = t1;
-        *reinterpret_cast<unsigned short *>(xterms + xstride + at * 2) = t2;
-        *reinterpret_cast<unsigned short *>(xterms + 2 * xstride + at * 2) = t3;
+        const __half h1 = __float2half_rn(e[j]);
+        const float r1 = (e[j] - __half2float(h1)) * 2048.0f;
+        const __half h2 = __float2half_rn(r1);
+        const float r2 = (r1 - __half2float(h2)) * 2048.0f;
+        t1 = __half_as_ushort(h1);
+        t2 = __half_as_ushort(h2);
+        t3 = __half_as_ushort(__float2half_rn(r2));
+        *reinterpret_cast<unsigned short *>(xterms + i * 2) = t1;
+        *reinterpret_cast<unsigned short *>(xterms + xstride + i * 2) = t2;
+        *reinterpret_cast<unsigned short *>(xterms + 2 * xstride + i * 2) = t3;
       }
     }
     if (p.norm_w) {
@@ -343,8 +315,8 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
     }
   }
   /* how the three columns of results add up to the product with x */
-  const float m0 = t == 0 ? 1.0f : (t == 1 ? (FP8 ? 1.0f / 4194304.0f : 1.0f) : 0.0f);
-  const float m1 = t == 0 ? (FP8 ? 1.0f / 2048.0f : 1.0f) : 0.0f;
+  const float m0 = t == 0 ? 1.0f : (t == 1 ? 1.0f / 4194304.0f : 0.0f);
+  const float m1 = t == 0 ? 1.0f / 2048.0f : 0.0f;
   const unsigned char *xb = xterms + (g < 3 ? g : 0) * xstride;
 
   int c_stage = 0, consumed = 0;
@@ -367,7 +339,7 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
       int item = tile * 8 + g;
       if (item >= p.items)
         item = p.items - 1;
-      const ItemRows mine = item_rows<W, EPI>(p, item);
+      const ItemRows mine = item_rows<Fp8W, EPI>(p, item);
       const float *sc_lo = reinterpret_cast<const float *>(mine.sc0);
       const float *sc_hi = reinterpret_cast<const float *>(mine.r1 ? mine.sc1 : mine.sc0);
       for (int ks = ks0; ks < ks1; ++ks) {
@@ -380,87 +352,43 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
           gave_up = true;
         }
         const unsigned char *st = my_ring + c_stage * STAGE_CODES_BYTES;
-        const unsigned char *ssc = my_scales + c_stage * F::scale_bytes;
-        (void)ssc;
         ++consumed;
         if (++c_stage == stages) {
           c_stage = 0;
           c_phase ^= 1;
         }
-        if (FP8) {
-          float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-          for (int grp = 0; grp < 2; ++grp) {
-            /* 16-byte chunk c of box row g sits at chunk c ^ g (128-byte swizzle) */
-            const int at = g * 128 + (((grp * 4 + t) ^ g) << 4);
-            const uint4 al = *reinterpret_cast<const uint4 *>(st + at);
-            const uint4 ah = *reinterpret_cast<const uint4 *>(st + 1024 + at);
-            uint4 b01 = make_uint4(0, 0, 0, 0), b23 = b01;
-            if (g < 3) {
-              const uint4 *bp = reinterpret_cast<const uint4 *>(
-                  xb + ((int64_t)ks * 128 + grp * 64 + t * 16) * 2);
-              b01 = bp[0];
-              b23 = bp[1];
-            }
-            const uint32_t wl[4] = {al.x, al.y, al.z, al.w};
-            const uint32_t wh[4] = {ah.x, ah.y, ah.z, ah.w};
-            const uint32_t bw[8] = {b01.x, b01.y, b01.z, b01.w,
-                                    b23.x, b23.y, b23.z, b23.w};
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              const uint32_t a[4] = {fp8x2_to_f16x2<false>(wl[m]),
-                                     fp8x2_to_f16x2<false>(wh[m]),
-                                     fp8x2_to_f16x2<true>(wl[m]),
-                                     fp8x2_to_f16x2<true>(wh[m])};
-              mma_f16(c, a, bw[2 * m], bw[2 * m + 1]);
-            }
+        for (int grp = 0; grp < 2; ++grp) {
+          /* 16-byte chunk c of box row g sits at chunk c ^ g (128-byte swizzle) */
+          const int at = g * 128 + (((grp * 4 + t) ^ g) << 4);
+          const uint4 al = *reinterpret_cast<const uint4 *>(st + at);
+          const uint4 ah = *reinterpret_cast<const uint4 *>(st + 1024 + at);
+          uint4 b01 = make_uint4(0, 0, 0, 0), b23 = b01;
+          if (g < 3) {
+            const uint4 *bp = reinterpret_cast<const uint4 *>(
+                xb + ((int64_t)ks * 128 + grp * 64 + t * 16) * 2);
+            b01 = bp[0];
+            b23 = bp[1];
           }
-          const float s_lo = __ldg(sc_lo + ks), s_hi = __ldg(sc_hi + ks);
-          lo0 = fmaf(s_lo, c[0], lo0);
-          lo1 = fmaf(s_lo, c[1], lo1);
-          hi0 = fmaf(s_hi, c[2], hi0);
-          hi1 = fmaf(s_hi, c[3], hi1);
-        } else {
-          const uint4 sl = *reinterpret_cast<const uint4 *>(ssc + g * 16);
-          const uint4 sh = *reinterpret_cast<const uint4 *>(ssc + 128 + g * 16);
-          const uint32_t slw[4] = {sl.x, sl.y, sl.z, sl.w};
-          const uint32_t shw[4] = {sh.x, sh.y, sh.z, sh.w};
+          const uint32_t wl[4] = {al.x, al.y, al.z, al.w};
+          const uint32_t wh[4] = {ah.x, ah.y, ah.z, ah.w};
+          const uint32_t bw[8] = {b01.x, b01.y, b01.z, b01.w,
+                                  b23.x, b23.y, b23.z, b23.w};
 #pragma unroll
-          for (int b = 0; b < 8; ++b) {
-            const int at = g * 128 + ((b ^ g) << 4) + 4 * t;
-            const uint32_t wl = *reinterpret_cast<const uint32_t *>(st + at);
-            const uint32_t wh = *reinterpret_cast<const uint32_t *>(st + 1024 + at);
-            uint4 bx = make_uint4(0, 0, 0, 0);
-            if (g < 3)
-              bx = *reinterpret_cast<const uint4 *>(
-                  xb + ((int64_t)ks * 256 + 32 * b + 8 * t) * 2);
-            /* a nibble OR-ed into 0x4300 is the bf16 128 + code; less 136 it
-               is code - 8, exactly */
-            constexpr uint32_t MAGIC = 0x43004300u, OFF = 0x43084308u, M = 0x000F000Fu;
-            const uint32_t l0 = sub_bf16x2((wl & M) | MAGIC, OFF);
-            const uint32_t l1 = sub_bf16x2(((wl >> 4) & M) | MAGIC, OFF);
-            const uint32_t l2 = sub_bf16x2(((wl >> 8) & M) | MAGIC, OFF);
-            const uint32_t l3 = sub_bf16x2(((wl >> 12) & M) | MAGIC, OFF);
-            const uint32_t h0 = sub_bf16x2((wh & M) | MAGIC, OFF);
-            const uint32_t h1 = sub_bf16x2(((wh >> 4) & M) | MAGIC, OFF);
-            const uint32_t h2 = sub_bf16x2(((wh >> 8) & M) | MAGIC, OFF);
-            const uint32_t h3 = sub_bf16x2(((wh >> 12) & M) | MAGIC, OFF);
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            const uint32_t a0[4] = {l0, h0, l1, h1};
-            mma_bf16(c, a0, bx.x, bx.y);
-            const uint32_t a1[4] = {l2, h2, l3, h3};
-            mma_bf16(c, a1, bx.z, bx.w);
-            const uint32_t pl = slw[b >> 1], ph = shw[b >> 1];
-            const float s_lo = __half2float(
-                __ushort_as_half((unsigned short)((b & 1) ? pl >> 16 : pl & 0xffffu)));
-            const float s_hi = __half2float(
-                __ushort_as_half((unsigned short)((b & 1) ? ph >> 16 : ph & 0xffffu)));
-            lo0 = fmaf(s_lo, c[0], lo0);
-            lo1 = fmaf(s_lo, c[1], lo1);
-            hi0 = fmaf(s_hi, c[2], hi0);
-            hi1 = fmaf(s_hi, c[3], hi1);
+          for (int m = 0; m < 4; ++m) {
+            const uint32_t a[4] = {fp8x2_to_f16x2<false>(wl[m]),
+                                   fp8x2_to_f16x2<false>(wh[m]),
+                                   fp8x2_to_f16x2<true>(wl[m]),
+                                   fp8x2_to_f16x2<true>(wh[m])};
+            mma_f16(c, a, bw[2 * m], bw[2 * m + 1]);
           }
         }
+        const float s_lo = __ldg(sc_lo + ks), s_hi = __ldg(sc_hi + ks);
+        lo0 = fmaf(s_lo, c[0], lo0);
+        lo1 = fmaf(s_lo, c[1], lo1);
+        hi0 = fmaf(s_hi, c[2], hi0);
+        hi1 = fmaf(s_hi, c[3], hi1);
         __syncwarp(); /* every lane has read the stage: it may be filled again */
         issue_next();
       }
@@ -501,23 +429,20 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
 
 /* nullptr: launched; "": this projection is not for this kernel (the caller
    takes the other one); anything else: an error. */
-template <typename W, int EPI>
+template <int EPI>
 const char *launch_quant_mma(RowDotParams &p, cudaStream_t stream) {
-  typedef QFmt<W> F;
   static const bool wanted = [] {
     const char *e = getenv("VXB_QUANT_MMA");
     return !(e && e[0] == '0');
   }();
-  constexpr bool FP8 = F::codes == 128;
-  if (!wanted || p.batch != 1 || p.expert_ids || p.items < 1 || p.cols % F::codes != 0 ||
-      p.cols % 4 != 0)
+  if (!wanted || p.batch != 1 || p.expert_ids || p.items < 1 || p.cols % STEP_COLS != 0)
     return "";
   if (EPI == EPI_QKV &&
       (p.rope_mode != 0 || p.w1 || p.w2 || (p.head_dim / 2) % 8 != 0))
     return "";
   QuantPlan plan;
   plan.tiles = (p.items + 7) / 8;
-  plan.ksteps = p.cols / F::codes;
+  plan.ksteps = p.cols / STEP_COLS;
   const int blocks = sm_count();
   plan.split = 1;
   while (plan.split < 16 && 2 * plan.split <= plan.ksteps &&
@@ -530,60 +455,42 @@ const char *launch_quant_mma(RowDotParams &p, cudaStream_t stream) {
     warps = WARPS;
   if (warps < 4)
     warps = 4 > plan.split ? 4 : plan.split; /* enough threads to stage x */
-  const size_t xbytes = 3 * (size_t)x_term_stride(p.cols, F::x_pad);
+  const size_t xbytes = 3 * (size_t)x_term_stride(p.cols, X_PAD);
   const size_t budget = 223 * 1024;
-  auto ring_of = [](int stages) { /* as the kernel lays it out */
-    return (size_t)((stages * (STAGE_CODES_BYTES + F::scale_bytes) + 1023) & ~1023);
-  };
   int stages = MAX_STAGES;
-  while (stages > 2 && xbytes + warps * ring_of(stages) > budget)
+  while (stages > 2 && xbytes + (size_t)warps * stages * STAGE_CODES_BYTES > budget)
     --stages;
-  if (xbytes + warps * ring_of(stages) > budget)
+  if (xbytes + (size_t)warps * stages * STAGE_CODES_BYTES > budget)
     return "";
   plan.warps = warps;
   plan.stages = stages;
-  const size_t smem = 1024 + warps * ring_of(stages) + xbytes;
+  const size_t smem = 1024 + (size_t)warps * stages * STAGE_CODES_BYTES + xbytes;
   /* the rows of the tiles' r0 and r1 halves as two maps (see item_rows) */
-  const uint64_t rb = (uint64_t)p.cols / PerWord<W>::n * 16; /* bytes of a row */
-  const uint64_t sb = (uint64_t)p.cols / 16;                 /* Q4_0: of its scales */
-  const char *w0 = (const char *)p.w0, *s0 = (const char *)p.s0 + p.row_base * sb;
-  CUtensorMap ma, mb, msa, msb;
+  const uint64_t rb = (uint64_t)p.cols; /* bytes of a row */
+  const char *w0 = (const char *)p.w0;
+  CUtensorMap ma, mb;
   bool ok;
   if (EPI == EPI_SWIGLU) {
     ok = make_byte_map(&ma, w0, rb, p.rows, rb, 128, true) &&
          make_byte_map(&mb, p.w1 ? (const char *)p.w1 : w0 + p.rows * rb, rb, p.rows, rb,
                        128, true);
-    if (ok && !FP8)
-      ok = make_byte_map(&msa, s0, sb, p.rows, sb, 16, false) &&
-           make_byte_map(&msb, p.w1 ? (const char *)p.s1 : s0 + p.rows * sb, sb, p.rows,
-                         sb, 16, false);
   } else if (EPI == EPI_QKV) {
     const uint64_t all = (uint64_t)(p.q_heads + 2 * p.kv_heads) * p.head_dim;
     ok = make_byte_map(&ma, w0, rb, all, rb, 128, true);
     mb = ma;
-    if (ok && !FP8) {
-      ok = make_byte_map(&msa, s0, sb, all, sb, 16, false);
-      msb = msa;
-    }
   } else {
     if (p.rows < 2)
       return "";
     ok = make_byte_map(&ma, w0, rb, (p.rows + 1) / 2, 2 * rb, 128, true) &&
          make_byte_map(&mb, w0 + rb, rb, p.rows / 2, 2 * rb, 128, true);
-    if (ok && !FP8)
-      ok = make_byte_map(&msa, s0, sb, (p.rows + 1) / 2, 2 * sb, 16, false) &&
-           make_byte_map(&msb, s0 + sb, sb, p.rows / 2, 2 * sb, 16, false);
   }
   if (!ok)
     return "";
-  if (FP8)
-    msa = msb = ma;
-  auto kernel = quant_mma_kernel<W, EPI>;
+  auto kernel = quant_mma_kernel<EPI>;
   if (allow_dynamic_smem((const void *)kernel, 224 * 1024) != cudaSuccess)
-    return "a quantised projection could not get its shared memory on this GPU";
-  launch_chained(kernel, dim3(blocks), dim3(plan.warps * 32), smem, stream, p, plan, ma, mb,
-                 msa, msb);
-  return check_launch("a quantised projection launch");
+    return "an fp8 projection could not get its shared memory on this GPU";
+  launch_chained(kernel, dim3(blocks), dim3(plan.warps * 32), smem, stream, p, plan, ma, mb);
+  return check_launch("an fp8 projection launch");
 }
 
 #endif /* VXB_ROWDOT_QUANT_MMA_CUH */
