@@ -246,28 +246,51 @@ attention_unit(const AttnArgs &a, int split_idx, int y, int b, int warp,
         d[j] = fmaf(qv[h].z, kv[j].z, d[j]);
         d[j] = fmaf(qv[h].w, kv[j].w, d[j]);
       }
+      /* The NB sums over the lanes: a lane keeps half of what it has, the positions whose
+         number has its bit, and gives the others away, until it has one sum; what it
+         then does for its position is done once and not by every lane. */
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+      for (int o = 16, n = NB / 2; n > 0; o >>= 1, n >>= 1) {
+        const bool upper = lane & o;
 #pragma unroll
-        for (int j = 0; j < NB; ++j)
-          d[j] += __shfl_xor_sync(0xffffffffu, d[j], o);
+        for (int i = 0; i < n; ++i) {
+          const float give = upper ? d[i] : d[n + i];
+          d[i] = (upper ? d[n + i] : d[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+#pragma unroll
+      for (int o = 16 / NB; o > 0; o >>= 1)
+        d[0] += __shfl_xor_sync(0xffffffffu, d[0], o);
+      const bool here = t0 + lane / (32 / NB) * ATT_WARPS < t_end;
+      const float s = here ? d[0] * scale : -3.0e38f;
+      float mn = s;
+#pragma unroll
+      for (int o = 16; o >= 32 / NB; o >>= 1)
+        mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mn = fmaxf(m[h], mn);
+      const float fix = expf(m[h] - mn);
+      const float mine = here ? expf(s - mn) : 0.0f;
+      m[h] = mn;
+      l[h] = l[h] * fix + mine; /* of this lane's positions */
+      acc[h].x *= fix;
+      acc[h].y *= fix;
+      acc[h].z *= fix;
+      acc[h].w *= fix;
 #pragma unroll
       for (int j = 0; j < NB; ++j) {
-        if (t0 + j * ATT_WARPS >= t_end)
-          continue;
-        const float s = d[j] * scale;
-        const float mn = fmaxf(m[h], s);
-        const float fix = expf(m[h] - mn);
-        const float pw = expf(s - mn);
-        l[h] = l[h] * fix + pw;
-        acc[h].x = acc[h].x * fix + pw * vv[j].x;
-        acc[h].y = acc[h].y * fix + pw * vv[j].y;
-        acc[h].z = acc[h].z * fix + pw * vv[j].z;
-        acc[h].w = acc[h].w * fix + pw * vv[j].w;
-        m[h] = mn;
+        const float pw = __shfl_sync(0xffffffffu, mine, j * (32 / NB));
+        acc[h].x = fmaf(pw, vv[j].x, acc[h].x);
+        acc[h].y = fmaf(pw, vv[j].y, acc[h].y);
+        acc[h].z = fmaf(pw, vv[j].z, acc[h].z);
+        acc[h].w = fmaf(pw, vv[j].w, acc[h].w);
       }
     }
   }
+#pragma unroll
+  for (int h = 0; h < GH; ++h)
+#pragma unroll
+    for (int o = 16; o >= 32 / NB; o >>= 1)
+      l[h] += __shfl_xor_sync(0xffffffffu, l[h], o);
 
   /* ---- merge the warps, in warp order ---- */
   float (&sm_m)[ATT_WARPS][GH] = sh.m;
