@@ -58,6 +58,23 @@ inline cudaError_t allow_dynamic_smem(const void *kernel, int bytes) {
   return e;
 }
 
+/* The kernel asks for all of an SM's memory as shared memory. An SM divides anew between
+   L1 and shared memory only when it is empty: a kernel with another wish than the one
+   before does not start beside it. Once per kernel and device, as above. */
+inline void prefer_shared_memory(const void *kernel) {
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, bool> asked;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess)
+    return;
+  std::lock_guard<std::mutex> lock(mu);
+  bool &done = asked[std::make_pair(kernel, dev)];
+  if (!done)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         cudaSharedmemCarveoutMaxShared);
+  done = true;
+}
+
 inline bool chain_enabled() {
   static const bool on = [] {
     const char *v = getenv("VXB_PDL");

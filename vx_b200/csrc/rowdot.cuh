@@ -17,6 +17,7 @@
 #include <cuda_fp16.h>
 
 #include <cstdio>
+#include <algorithm>
 #include <climits>
 #include <cstdlib>
 

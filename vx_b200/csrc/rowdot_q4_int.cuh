@@ -24,15 +24,18 @@
  * tiles; its loads (cp.async, 16 rows x 128 bytes and their scales, into a ring of its
  * own) run ahead through all of them, and the first ones start before the kernel that
  * makes x has finished.  The warps' sums meet in shared memory once, when the block's
- * tiles are done.  Eight warps and at most 113 KB, so that the block of the next
- * projection is resident, and its ring full, before this one leaves the SM.  (12 warps of
- * 80 registers: the 7B-shaped step 11 % longer; 16 of 64, which spill: 36 %.)
+ * tiles are done.  Eight warps, and at most half of an SM's registers and shared memory, so
+ * that the block of the next projection is resident, and its ring full, before this one
+ * leaves the SM.  (Slower, us a layer where this takes 44.5: one block of 16 warps an SM
+ * 49.3, two of 12 warps 49.8, L2 asked for the rest of a block's rows at its start 58.)
  *
- * What bounds it: a long launch runs at 5.0 to 5.5 TB/s of weights (90000 x 4096, 38 to 42
- * us; 81 before), short ones at that plus the 3 us between the end of the kernel before
- * and the first product (its signal, x, the bytes of x).  Back to back in a graph, us:
- * 12288 x 4096 7.8 (13.6 on bf16 mma.sync), 4096 x 4096 4.1 (6.7), 22016 x 4096 11.4
- * (23.1), 4096 x 11008 8.6 (13.3).
+ * What bounds it: alone, 90000 x 4096 runs at 5.0 to 5.5 TB/s of weights (38 to 42 us; 81
+ * before).  In a layer, a projection takes 1.1 us from the end of the kernel before to its
+ * signal, 1.1 (4096 columns) to 3.2 (11008) for x, and then as long as its instructions
+ * take: eight warps issue half the time, 8.6 us for the 22016 x 4096 of gate/up, of which
+ * HBM would take 7.7.  Back to back in a graph, us: 12288 x 4096 7.8 to 9.3 (13.6 on bf16
+ * mma.sync), 4096 x 4096 4.1 to 5.6 (6.7), 22016 x 4096 11.4 to 12.7 (23.1), 4096 x 11008
+ * 8.6 to 10.3 (13.3).
  */
 #ifndef VXB_ROWDOT_Q4_INT_CUH
 #define VXB_ROWDOT_Q4_INT_CUH
@@ -114,7 +117,7 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
      a fixed distance behind those of the warp's tile before (of q, k and v: until the
      half of a head ends). ---- */
   const int64_t row_bytes = cols / 2, scale_bytes = cols / 16;
-  const int half = EPI == EPI_QKV ? p.head_dim / 2 : 0;
+  const int half = EPI == EPI_QKV ? p.head_dim / 2 : 1;
   struct Row {
     int row0, row1; /* of w0, of w1 or w0 */
     int in_half;    /* q, k and v */
@@ -215,6 +218,9 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
   for (int s = 0; s < STAGES; ++s)
     issue_next();
   chain_release();
+  if (p.norm_w) /* nor do the norm's gains, which come from HBM once a step */
+    for (int at = threadIdx.x * 128; at < cols * (p.norm_bf16 ? 2 : 4); at += I_WARPS * 32 * 128)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)p.norm_w + at));
   chain_wait();
 
   /* ---- x, times the norm's gains if any, as whole numbers: a thread takes eight
@@ -439,23 +445,29 @@ template <int EPI> const char *launch_q4_int(RowDotParams &p, cudaStream_t strea
       plan.slices = n;
     }
   }
-  /* two blocks on an SM, with their 1 KB each; one */
-  const size_t half = 113 * 1024;
-  const int most = 226 * 1024;
+  /* Two projections one after another share an SM's 228 KB, two blocks of one projection
+     must not: another SM would be without. (Attention leaves SMs uneven. With 111 KB for
+     all, gate/up took 14.7 us on SMs with two blocks, 8.5 on those with one, and the SMs
+     with none waited: 58 us a layer of the 7B shape at 1000 positions, so 44.5.) So what
+     follows attention or gate/up takes 115 KB, q/k/v and gate/up at most 111. */
+  const size_t floor_bytes = EPI == EPI_QKV || EPI == EPI_SWIGLU ? 0 : 115 * 1024;
+  const size_t share = EPI == EPI_QKV || EPI == EPI_SWIGLU ? 111 * 1024 : 115 * 1024;
+  const size_t most = 226 * 1024;
   auto go = [&](auto kernel, size_t smem) -> const char * {
-    if (allow_dynamic_smem((const void *)kernel, most) != cudaSuccess)
+    if (allow_dynamic_smem((const void *)kernel, (int)most) != cudaSuccess)
       return "a Q4_0 projection could not get its shared memory on this GPU";
-    launch_chained(kernel, dim3(blocks), dim3(I_WARPS * 32), smem, stream, p, plan);
+    prefer_shared_memory((const void *)kernel);
+    launch_chained(kernel, dim3(blocks), dim3(I_WARPS * 32), std::max(smem, floor_bytes), stream, p,
+                   plan);
     return check_launch("a Q4_0 projection launch");
   };
   plan.round = 16;
-  if (q4_int_smem(3, p.cols, plan) > half)
+  if (q4_int_smem(3, p.cols, plan) > share)
     plan.round = 8;
-  const size_t four = q4_int_smem(4, p.cols, plan);
-  const size_t three = q4_int_smem(3, p.cols, plan);
-  if (three > (size_t)most)
+  const size_t four = q4_int_smem(4, p.cols, plan), three = q4_int_smem(3, p.cols, plan);
+  if (three > most)
     return "";
-  if (four <= half || (three > half && four <= (size_t)most))
+  if (four <= share || (three > share && four <= most))
     return go(q4_int_kernel<EPI, 4>, four);
   return go(q4_int_kernel<EPI, 3>, three);
 }
