@@ -319,19 +319,27 @@ attention_unit(const AttnArgs &a, int split_idx, int y, int b, int warp,
     if (warp == 0) {
       /* the block's part, left in row 0 of its own shared arrays */
       for (int h = 0; h < nh; ++h) {
-        float big = -3.0e38f;
-        for (int w = 0; w < ATT_WARPS; ++w)
-          big = fmaxf(big, sm_m[w][h]);
-        float total = 0.0f;
+        /* lane w: the factor of warp w's part */
+        const float mine = lane < ATT_WARPS ? sm_m[lane][h] : -3.0e38f;
+        const float big = warp_max(mine);
+        const float part = lane < ATT_WARPS ? expf(mine - big) : 0.0f;
+        const float total = warp_sum(lane < ATT_WARPS ? part * sm_l[lane][h] : 0.0f);
         float4 o = make_float4(0, 0, 0, 0);
+#pragma unroll 4
         for (int w = 0; w < ATT_WARPS; ++w) {
-          const float f = expf(sm_m[w][h] - big);
-          total += f * sm_l[w][h];
+          const float f = __shfl_sync(0xffffffffu, part, w);
           if (active) {
             const float4 v =
                 *reinterpret_cast<const float4 *>(&sm_acc[w][h][lane * 4]);
             o.x += f * v.x; o.y += f * v.y; o.z += f * v.z; o.w += f * v.w;
           }
+        }
+        if (CL == 1) {
+          if (active)
+            *reinterpret_cast<float4 *>(a.out + ((int64_t)b * a.q_heads + h0 + h) * hd +
+                                        lane * 4) =
+                make_float4(o.x / total, o.y / total, o.z / total, o.w / total);
+          continue;
         }
         __syncwarp();
         if (active)
@@ -342,6 +350,8 @@ attention_unit(const AttnArgs &a, int split_idx, int y, int b, int warp,
         }
       }
     }
+    if (CL == 1)
+      return;
     cluster.sync();
     if (cluster.block_rank() == 0) {
       /* block 0 merges the runs in order: warp h takes head h */
