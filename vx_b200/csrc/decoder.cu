@@ -431,7 +431,7 @@ void record_step(vx_decoder *d, int max_pos) {
                      int rows, int cols, const float *x, const void *norm_w,
                      float *y, int64_t y_stride, const void *bias, int layer,
                      const char *what, bool terms_ready = false,
-                     bool leave_terms = false) {
+                     bool leave_terms = false, const void *next_norm = nullptr) {
     vxb::BatchedProj bp{};
     bp.mode = mode;
     bp.w0 = w0;
@@ -460,14 +460,17 @@ void record_step(vx_decoder *d, int max_pos) {
     bp.scratch = d->mma_scratch;
     bp.x_terms_ready = terms_ready;
     bp.next_terms = leave_terms;
+    bp.next_norm_w = next_norm;
     need(vxb::batched_proj(bp, s), what);
     launches += terms_ready ? 2 : 3;
   };
+  /* a residual projection leaves the next one's input, normalised */
+  const bool norm_left = d->mma && vxb::batched_proj_leaves_norm(c.dim);
   for (int l = 0; l < c.n_layers; ++l) {
     if (d->mma) {
       batched(4, d->wq[l], d->wk[l], d->wv[l], (d->q_local + 2 * d->kv_local) * hd,
               c.dim, d->x, d->attn_norm[l], d->q, (int64_t)d->q_local * hd,
-              d->bqkv[l], l, "q/k/v");
+              d->bqkv[l], l, "q/k/v", norm_left && l > 0);
       vxb::AttnArgs ab{};
       ab.q = d->q;
       ab.k_cache = d->k_cache + l * d->cache_layer_stride;
@@ -487,13 +490,16 @@ void record_step(vx_decoder *d, int max_pos) {
       need(vxb::attention_decode(ab, s), "attention");
       ++launches;
       batched(1, d->wo[l], nullptr, nullptr, c.dim, d->q_local * hd, d->att,
-              nullptr, d->x, c.dim, nullptr, l, "the output projection");
+              nullptr, d->x, c.dim, nullptr, l, "the output projection", false,
+              norm_left, norm_left ? d->ffn_norm[l] : nullptr);
       /* SwiGLU's finishing kernel leaves the down projection's input as terms */
       batched(3, d->w_gate[l], d->w_up[l], nullptr, d->hidden_local, c.dim, d->x,
-              d->ffn_norm[l], d->h, d->hidden_local, nullptr, l, "gate/up", false,
+              d->ffn_norm[l], d->h, d->hidden_local, nullptr, l, "gate/up", norm_left,
               true);
+      const void *next = l + 1 < c.n_layers ? d->attn_norm[l + 1] : d->final_norm;
       batched(1, d->w_down[l], nullptr, nullptr, c.dim, d->hidden_local, d->h,
-              nullptr, d->x, c.dim, nullptr, l, "the down projection", true);
+              nullptr, d->x, c.dim, nullptr, l, "the down projection", true, norm_left,
+              norm_left ? next : nullptr);
       continue;
     }
     vxb::QkvArgs qa{};
@@ -602,7 +608,8 @@ void record_step(vx_decoder *d, int max_pos) {
 
   if (d->mma) {
     batched(0, d->lm_head, nullptr, nullptr, d->vocab_local, c.dim, d->x,
-            d->final_norm, d->logits, d->vocab_local, nullptr, 0, "the logits");
+            d->final_norm, d->logits, d->vocab_local, nullptr, 0, "the logits",
+            norm_left && c.n_layers > 0);
   } else {
   vxb::MatvecArgs la{};
   la.w = d->lm_head;

@@ -277,6 +277,7 @@ rowdot_kernel(const RowDotParams p) {
     ld_s0 = it.sc0;
     ld_s1 = it.r1 ? it.sc1 : it.sc0;
   }
+  const uint64_t policy = ptx::evict_first();
   auto issue_next = [&]() {
     if (ld_u >= units)
       return;
@@ -286,8 +287,8 @@ rowdot_kernel(const RowDotParams p) {
       uint64_t *bar = &bars[warp][ld_stage];
       const int sbytes = ring_scales ? bytes / 8 : 0;
       ptx::mbar_expect_tx(bar, 2 * bytes + 2 * sbytes);
-      ptx::bulk_load(dst, ld_r0 + ld_ch * CHUNK_BYTES, bytes, bar);
-      ptx::bulk_load(dst + CHUNK_BYTES, ld_r1 + ld_ch * CHUNK_BYTES, bytes, bar);
+      ptx::bulk_load(dst, ld_r0 + ld_ch * CHUNK_BYTES, bytes, bar, policy);
+      ptx::bulk_load(dst + CHUNK_BYTES, ld_r1 + ld_ch * CHUNK_BYTES, bytes, bar, policy);
       if (ring_scales) {
         ptx::bulk_load(dst + 2 * CHUNK_BYTES, ld_s0 + ld_ch * SC, sbytes, bar);
         ptx::bulk_load(dst + 2 * CHUNK_BYTES + SC, ld_s1 + ld_ch * SC, sbytes, bar);

@@ -50,8 +50,9 @@ struct Q4IntPlan {
   int round;  /* tiles between two meetings of the warps: 8 or 16 */
 };
 
-__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src)
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, uint64_t policy) {
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint.L2::128B [%0], [%1], 16, %2;" ::"r"(dst),
+               "l"(src), "l"(policy)
                : "memory");
 }
 
@@ -184,19 +185,20 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
   const uint32_t to1 = ring_at + ((lane >> 3) + 4) * 128 +
                        (((lane & 7) ^ ((lane >> 3) + 4)) << 4);
   const uint32_t to_scale = ring_at + I_CODE_BYTES + lane * 16;
+  const uint64_t policy = ptx::evict_first();
   auto issue_next = [&]() {
     if (ld_tile < tiles) {
       const uint32_t at = ld_stage * I_STAGE_BYTES;
       if (have[0])
-        copy16_async(to0 + at, src[0]);
+        copy16_async(to0 + at, src[0], policy);
       if (have[1])
-        copy16_async(to1 + at, src[1]);
+        copy16_async(to1 + at, src[1], policy);
       if (have[2])
-        copy16_async(to0 + at + 1024, src[2]);
+        copy16_async(to0 + at + 1024, src[2], policy);
       if (have[3])
-        copy16_async(to1 + at + 1024, src[3]);
+        copy16_async(to1 + at + 1024, src[3], policy);
       if (have_scale)
-        copy16_async(to_scale + at, src_scale);
+        copy16_async(to_scale + at, src_scale, policy);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         src[i] += 128;

@@ -31,6 +31,7 @@
 #include "launch.cuh"
 #include "ptx.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <cstdio>
@@ -203,6 +204,7 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
           cur_item += gridDim.x;
         }
       };
+      const uint64_t policy = ptx::evict_first();
       auto load_weights = [&](int s, int kb) {
         uint8_t *sa = smem + s * stage_bytes;
         ptx::mbar_expect_tx(&bars->full[s], A_BYTES + b_bytes);
@@ -211,7 +213,7 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
           const CUtensorMap *m = which[h] == 0 ? &map_w0
                                  : which[h] == 1 ? &map_w1 : &map_w2;
           ptx::tma_load_2d(sa + h * (A_BYTES / 2), m, kb * BK, row0[h],
-                           &bars->full[s]);
+                           &bars->full[s], policy);
         }
       };
       /* The weights do not depend on the kernel before; the x terms do: the
@@ -351,51 +353,90 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
   }
 }
 
-/* The runs of K added in run order (so the result does not depend on
-   timing), then the projection's own epilogue. One thread per sequence and
-   per output row (modes 0, 1), SwiGLU unit (mode 3) or rotation pair (mode 4). */
+/* The runs of K of `N` neighbouring padded rows of sequence b, added in run order (so the
+   result does not depend on timing). */
+template <int N> struct Few {
+  float v[N];
+};
+template <int N>
+__device__ __forceinline__ Few<N> sum_of_runs(const MmaParams &p, int b, int64_t row) {
+  const int64_t padded_rows = (int64_t)p.tiles * TM;
+  const float *at = p.partials + (int64_t)b * padded_rows + row;
+  float2 two[N == 2 ? 16 : 1];
+  float one[N == 1 ? 16 : 1];
+#pragma unroll
+  for (int s = 0; s < 16; ++s) {
+    const float *run = at + (int64_t)s * p.batch * padded_rows;
+    if (N == 2)
+      two[s % (N == 2 ? 16 : 1)] =
+          s < p.splits ? __ldcg(reinterpret_cast<const float2 *>(run)) : make_float2(0, 0);
+    else
+      one[s % (N == 1 ? 16 : 1)] = s < p.splits ? __ldcg(run) : 0.0f;
+  }
+  Few<N> t = {};
+#pragma unroll
+  for (int s = 0; s < 16; ++s)
+    if (s < p.splits) {
+      if (N == 2) {
+        t.v[0] += two[s % (N == 2 ? 16 : 1)].x;
+        t.v[N - 1] += two[s % (N == 2 ? 16 : 1)].y;
+      } else {
+        t.v[0] += one[s % (N == 1 ? 16 : 1)];
+      }
+    }
+  return t;
+}
+
+/* The sums of the runs, then the projection's own epilogue. A thread has N neighbouring
+   output rows of a sequence (modes 0, 1), SwiGLU units (mode 3) or rotation pairs (mode
+   4): with two the blocks of gate/up are resident at once beside those of the product. */
+template <int N>
 __global__ void __launch_bounds__(256)
 proj_finish_kernel(const MmaParams p) {
   chain_release();
-  chain_wait();
   const int B = p.batch;
-  const int64_t padded_rows = (int64_t)p.tiles * TM;
   const int per_seq = p.mode == 0 || p.mode == 1 ? p.rows : p.tiles * 64;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)per_seq * B)
+  const int64_t idx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * N;
+  const bool in = idx < (int64_t)per_seq * B;
+  const int b = in ? (int)(idx / per_seq) : 0, e = in ? (int)(idx - (int64_t)b * per_seq) : 0;
+  const int tile = e / 64, r = e - tile * 64;
+  /* positions and tables are of earlier steps and come from HBM: asked for first */
+  int pos = 0;
+  float c[N] = {}, sn[N] = {};
+  if (p.mode == 4 && in) {
+    pos = p.positions[b];
+    if (tile < p.q_heads + p.kv_heads)
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        c[i] = p.cos_t[(int64_t)pos * 64 + r + i];
+        sn[i] = p.sin_t[(int64_t)pos * 64 + r + i];
+      }
+  }
+  chain_wait();
+  if (!in)
     return;
-  const int b = (int)(idx / per_seq), e = (int)(idx - (int64_t)b * per_seq);
-  /* the value of padded row `row`, all runs */
-  auto total = [&](int64_t row) {
-    const float *at = p.partials + (int64_t)b * padded_rows + row;
-    float v[16];
-#pragma unroll
-    for (int s = 0; s < 16; ++s)
-      v[s] = s < p.splits ? __ldcg(at + (int64_t)s * B * padded_rows) : 0.0f;
-    float t = 0.0f;
-#pragma unroll
-    for (int s = 0; s < 16; ++s)
-      if (s < p.splits)
-        t += v[s];
-    return t;
-  };
   if (p.mode == 0 || p.mode == 1) {
     float *y = p.y + b * p.y_stride + e;
-    const float t = total(e);
-    *y = p.mode == 1 ? *y + t : t;
+    const Few<N> t = sum_of_runs<N>(p, b, e);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      y[i] = p.mode == 1 ? y[i] + t.v[i] : t.v[i];
     return;
   }
-  const int tile = e / 64, r = e - tile * 64;
-  const float lo = total((int64_t)tile * TM + r), hi = total((int64_t)tile * TM + r + 64);
+  const Few<N> lo = sum_of_runs<N>(p, b, (int64_t)tile * TM + r);
+  const Few<N> hi = sum_of_runs<N>(p, b, (int64_t)tile * TM + r + 64);
   if (p.mode == 3) {
-    if (e < p.rows) { /* nn_swiglu (nn.vx:169-209): g / (1 + e^-g) * u */
-      const float h = lo / (1.0f + expf(0.0f - lo)) * hi;
-      p.y[b * p.y_stride + e] = h;
+#pragma unroll
+    for (int i = 0; i < N; ++i) { /* nn_swiglu (nn.vx:169-209): g / (1 + e^-g) * u */
+      if (e + i >= p.rows)
+        break;
+      const float h = lo.v[i] / (1.0f + expf(0.0f - lo.v[i])) * hi.v[i];
+      p.y[b * p.y_stride + e + i] = h;
       if (p.terms) {
-        store_terms(p.terms, p.rows, B, b, e, h);
+        store_terms(p.terms, p.rows, B, b, e + i, h);
         if (b == 0)
           for (int row = 3 * B; row < p.terms_n; ++row)
-            p.terms[(int64_t)row * p.rows + e] = __float2bfloat16(0.0f);
+            p.terms[(int64_t)row * p.rows + e + i] = __float2bfloat16(0.0f);
       }
     }
     return;
@@ -406,26 +447,87 @@ proj_finish_kernel(const MmaParams p) {
   const int local = kind == 0 ? head
                     : kind == 1 ? head - p.q_heads
                                 : head - p.q_heads - p.kv_heads;
-  float va = lo, vb = hi;
-  if (p.bias) {
-    va += bf16_val(p.bias, (int64_t)head * 128 + r);
-    vb += bf16_val(p.bias, (int64_t)head * 128 + r + 64);
-  }
-  const int pos = p.positions[b];
-  if (kind == 2) {
-    float *vrow = p.v_cache + b * p.cache_batch_stride +
-                  ((int64_t)pos * p.kv_heads + local) * 128;
-    vrow[r] = va;
-    vrow[r + 64] = vb;
-    return;
-  }
-  const float c = p.cos_t[(int64_t)pos * 64 + r];
-  const float sn = p.sin_t[(int64_t)pos * 64 + r];
   float *dst = kind == 0 ? p.y + b * p.y_stride + (int64_t)local * 128
-                         : p.k_cache + b * p.cache_batch_stride +
+                         : (kind == 1 ? p.k_cache : p.v_cache) + b * p.cache_batch_stride +
                                ((int64_t)pos * p.kv_heads + local) * 128;
-  dst[r] = __fsub_rn(__fmul_rn(va, c), __fmul_rn(vb, sn));
-  dst[r + 64] = __fadd_rn(__fmul_rn(vb, c), __fmul_rn(va, sn));
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float va = lo.v[i], vb = hi.v[i];
+    if (p.bias) {
+      va += bf16_val(p.bias, (int64_t)head * 128 + r + i);
+      vb += bf16_val(p.bias, (int64_t)head * 128 + r + i + 64);
+    }
+    dst[r + i] = kind == 2 ? va : __fsub_rn(__fmul_rn(va, c[i]), __fmul_rn(vb, sn[i]));
+    dst[r + i + 64] = kind == 2 ? vb : __fadd_rn(__fmul_rn(vb, c[i]), __fmul_rn(va, sn[i]));
+  }
+}
+
+/* Mode 1 where an RMSNorm follows: y += the product, and the three terms of the
+   normalised y for the next projection.  A cluster of eight blocks a sequence, each an
+   eighth of its row; the sums of squares meet through distributed shared memory.  It takes
+   the place of a finishing kernel and of split3_kernel, 3.5 us each between two products
+   of a layer of 16 sequences. */
+constexpr int NORM_BLOCKS = 8, NORM_THREADS = 256;
+__global__ void __launch_bounds__(NORM_THREADS)
+add_norm_terms_kernel(const MmaParams p, const void *norm_w, float eps) {
+  __shared__ float red[NORM_THREADS / 32], sums;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  chain_release();
+  const int b = blockIdx.x / NORM_BLOCKS, rank = blockIdx.x % NORM_BLOCKS;
+  const int pairs = p.rows / 2;
+  const int first = (int)((int64_t)pairs * rank / NORM_BLOCKS);
+  const int last = (int)((int64_t)pairs * (rank + 1) / NORM_BLOCKS);
+  float2 *y = reinterpret_cast<float2 *>(p.y + b * p.y_stride);
+  chain_wait();
+  /* (rolled: straight-line code for eight pairs took 6 us, most of it its own way from
+     HBM, where the weights of a layer drive it out of L2) */
+  float ss = 0.0f;
+#pragma unroll 1
+  for (int i = first + threadIdx.x; i < last; i += NORM_THREADS) {
+    const float2 old = y[i];
+    const Few<2> t = sum_of_runs<2>(p, b, 2 * (int64_t)i);
+    const float2 v = make_float2(old.x + t.v[0], old.y + t.v[1]);
+    y[i] = v;
+    ss = fmaf(v.x, v.x, ss);
+    ss = fmaf(v.y, v.y, ss);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0)
+    red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.0f;
+    for (int w = 0; w < NORM_THREADS / 32; ++w) /* fixed order */
+      t += red[w];
+    sums = t;
+  }
+  cluster.sync();
+  float total = 0.0f;
+#pragma unroll
+  for (int r = 0; r < NORM_BLOCKS; ++r) /* fixed order */
+    total += *cluster.map_shared_rank(&sums, r);
+  const float inv = 1.0f / sqrtf(total / (float)p.rows + eps);
+  const int B = p.batch;
+#pragma unroll 1
+  for (int i = first + threadIdx.x; i < last; i += NORM_THREADS) {
+    const float2 v = y[i]; /* this thread's own */
+    float a[2] = {v.x * inv * bf16_val(norm_w, 2 * i), v.y * inv * bf16_val(norm_w, 2 * i + 1)};
+    __nv_bfloat162 *to = reinterpret_cast<__nv_bfloat162 *>(p.terms);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const __nv_bfloat162 x = __floats2bfloat162_rn(a[0], a[1]);
+      to[(int64_t)(t * B + b) * pairs + i] = x;
+      a[0] -= __bfloat162float(x.x);
+      a[1] -= __bfloat162float(x.y);
+    }
+    if (b == 0)
+      for (int row = 3 * B; row < p.terms_n; ++row)
+        to[(int64_t)row * pairs + i] = __floats2bfloat162_rn(0.0f, 0.0f);
+  }
+  cluster.sync(); /* nobody leaves while another may still read its sum */
 }
 
 /* x (f32, optionally RMS-normalised first: nn_rms_norm, nn.vx:212-239) as three
@@ -524,6 +626,10 @@ const char *batched_proj_refusal(const BatchedProj &a) {
   return nullptr;
 }
 
+bool batched_proj_leaves_norm(int rows) {
+  return rows % 2 == 0;
+}
+
 size_t batched_proj_scratch_floats(int rows_max, int batch) {
   /* up to 16 runs of [batch][rows rounded up to 128] */
   return (size_t)16 * batch * ((rows_max + 127) / 128 * 128);
@@ -560,8 +666,12 @@ const char *batched_proj(const BatchedProj &a, cudaStream_t stream) {
   p.partials = a.scratch;
   p.terms = a.next_terms ? (__nv_bfloat16 *)a.xs : nullptr;
   p.terms_n = a.next_terms ? (3 * a.batch + 15) / 16 * 16 : 0;
-  if (a.next_terms && a.mode != 3)
-    return "only the SwiGLU projection can leave terms";
+  if (a.next_terms && a.mode != 3 && (a.mode != 1 || !a.next_norm_w))
+    return "only the SwiGLU and the residual projections can leave terms";
+  if (a.next_terms && a.mode == 1 &&
+      (!batched_proj_leaves_norm(a.rows) || a.y_stride % 2 != 0 ||
+       (((uintptr_t)a.y | (uintptr_t)a.xs) & 7)))
+    return "terms of a normalised row need pairs of values";
   int64_t rows0 = a.rows, rows1 = 0, rows2 = 0; /* rows of the three matrices */
   if (a.mode == 3) {
     p.tiles = a.rows / 64;
@@ -601,8 +711,14 @@ const char *batched_proj(const BatchedProj &a, cudaStream_t stream) {
                  m2, mx, p);
   const int64_t outputs =
       (int64_t)a.batch * (p.mode == 0 || p.mode == 1 ? p.rows : p.tiles * 64);
-  launch_chained(proj_finish_kernel, dim3((unsigned)((outputs + 255) / 256)),
-                 dim3(256), 0, stream, p);
+  auto blocks = [&](int per) { return dim3((unsigned)((outputs + 256 * per - 1) / (256 * per))); };
+  if (p.mode == 1 && a.next_terms)
+    launch_chained_cluster(add_norm_terms_kernel, dim3(NORM_BLOCKS * a.batch),
+                           dim3(NORM_THREADS), NORM_BLOCKS, stream, p, a.next_norm_w, a.eps);
+  else if (p.mode > 1 || a.rows % 2 == 0) /* a pair is of one sequence, and of one tile */
+    launch_chained(proj_finish_kernel<2>, blocks(2), dim3(256), 0, stream, p);
+  else
+    launch_chained(proj_finish_kernel<1>, blocks(1), dim3(256), 0, stream, p);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     static thread_local char msg[160];
