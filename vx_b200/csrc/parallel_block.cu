@@ -84,12 +84,10 @@ fan_finish_kernel(const float *partials, int splits, int t_count, int n,
                   int out_col) {
   chain_release();
   chain_wait();
-  const int per_row = n / 8;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)t_count * per_row)
+  const int r = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (r >= n)
     return;
-  const int64_t t = idx / per_row;
-  const int r = (int)(idx - t * per_row) * 8;
+  const int64_t t = blockIdx.x;
   const float4 lo = sum_runs4(partials, splits, t_count, n, t, r);
   const float4 hi = sum_runs4(partials, splits, t_count, n, t, r + 4);
   float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
@@ -223,9 +221,7 @@ const char *rows_fan_finish(const float *partials, int splits, int t, int n,
                             int out_col, cudaStream_t stream) {
   if ((n | out.k_row | out.gate_row | out.up_row | out_cols | out_col) % 8 != 0)
     return "the parts of an input projection are multiples of 8 rows";
-  const int64_t count = (int64_t)t * (n / 8);
-  launch_chained(fan_finish_kernel, dim3((unsigned)((count + 255) / 256)), dim3(256), 0,
-                 stream, partials, splits, t, n, out, positions, q_out, q_stride,
+  launch_chained(fan_finish_kernel, dim3(t, (n / 8 + 255) / 256), dim3(256), 0, stream, partials, splits, t, n, out, positions, q_out, q_stride,
                  k_cache, (__nv_bfloat16 *)terms, out_cols, out_col);
   return check_launch("the parts of an input projection");
 }

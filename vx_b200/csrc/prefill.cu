@@ -343,6 +343,79 @@ residual_norm_kernel(__nv_bfloat16 *terms, float *x, const float *partials,
   }
 }
 
+/* The same for rows of whole quads, at most QUADS of them a thread, whose loads of a run are
+   in flight together. Value by value, a trip to L2 after another, 499 rows of 4096 took 28
+   us; so 10. */
+template <int QUADS>
+__global__ void __launch_bounds__(256)
+residual_norm_quads_kernel(__nv_bfloat16 *terms, float *x, const float *partials, int splits,
+                           int t_count, const NormGain w, int dim, float eps) {
+  __shared__ float red[8];
+  chain_release();
+  chain_wait();
+  const int64_t t = blockIdx.x;
+  float4 *xr = reinterpret_cast<float4 *>(x + t * dim);
+  const float4 *part = reinterpret_cast<const float4 *>(partials + t * dim);
+  const int64_t run = (int64_t)t_count * dim / 4;
+  const int quads = dim / 4;
+  float4 old[QUADS], v[QUADS];
+#pragma unroll
+  for (int k = 0; k < QUADS; ++k) {
+    const int i = threadIdx.x + k * 256;
+    old[k] = v[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (i < quads) {
+      old[k] = xr[i];
+      v[k] = part[i];
+    }
+  }
+#pragma unroll 2
+  for (int s = 1; s < splits; ++s) {
+    part += run;
+#pragma unroll
+    for (int k = 0; k < QUADS; ++k) {
+      const int i = threadIdx.x + k * 256;
+      if (i < quads) {
+        const float4 p = part[i];
+        v[k].x += p.x; v[k].y += p.y; v[k].z += p.z; v[k].w += p.w;
+      }
+    }
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < QUADS; ++k) {
+    const int i = threadIdx.x + k * 256;
+    v[k].x = old[k].x + v[k].x;
+    v[k].y = old[k].y + v[k].y;
+    v[k].z = old[k].z + v[k].z;
+    v[k].w = old[k].w + v[k].w;
+    if (i < quads)
+      xr[i] = v[k];
+    ss = fmaf(v[k].x, v[k].x, ss); /* zeros beyond the row */
+    ss = fmaf(v[k].y, v[k].y, ss);
+    ss = fmaf(v[k].z, v[k].z, ss);
+    ss = fmaf(v[k].w, v[k].w, ss);
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0)
+    red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float total = 0.0f;
+  for (int k = 0; k < 8; ++k) /* fixed order */
+    total += red[k];
+  const float inv = 1.0f / sqrtf(total / (float)(w.n ? w.n : dim) + eps);
+#pragma unroll
+  for (int k = 0; k < QUADS; ++k) {
+    const int i = threadIdx.x + k * 256;
+    if (i < quads) {
+      const float out[4] = {v[k].x * gain_at(w, 4 * i) * inv, v[k].y * gain_at(w, 4 * i + 1) * inv,
+                            v[k].z * gain_at(w, 4 * i + 2) * inv,
+                            v[k].w * gain_at(w, 4 * i + 3) * inv};
+      store_terms4(terms, dim, t, 4 * i, out);
+    }
+  }
+}
+
 /* After the q/k/v GEMM: bias, half-split RoPE (nn_rope_and_store,
    nn.vx:245-280), q to q_out[t], k and v to row first_pos + t of the cache.
    One thread per (position, head, pair i / i + hd/2). */
@@ -356,12 +429,11 @@ qkv_finish_kernel(const float *partials, int splits, int t_count, int q_heads,
   /* one thread per (position, head, four pairs i..i+3 / i + hd/2 ..) */
   const int half = hd / 2, quads = half / 4, heads = q_heads + 2 * kv_heads;
   const int64_t n = (int64_t)heads * hd;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)t_count * heads * quads)
+  const int idx = blockIdx.y * blockDim.x + threadIdx.x;
+  if (idx >= heads * quads)
     return;
-  const int i = (int)(idx % quads) * 4;
-  const int head = (int)((idx / quads) % heads);
-  const int64_t t = idx / ((int64_t)quads * heads);
+  const int head = idx / quads, i = (idx - head * quads) * 4;
+  const int64_t t = blockIdx.x;
   const int64_t ra = (int64_t)head * hd + i, rb = ra + half;
   float4 va = sum_runs4(partials, splits, t_count, n, t, ra);
   float4 vb = sum_runs4(partials, splits, t_count, n, t, rb);
@@ -417,12 +489,10 @@ swiglu_finish_kernel(__nv_bfloat16 *terms, const float *partials, int splits,
   chain_release();
   chain_wait();
   /* one thread per (position, eight consecutive rows): hidden % 8 == 0 */
-  const int per_row = hidden / 8;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)t_count * per_row)
+  const int r = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (r >= hidden)
     return;
-  const int64_t t = idx / per_row;
-  const int r = (int)(idx - t * per_row) * 8;
+  const int64_t t = blockIdx.x;
   const int64_t n = 2 * (int64_t)hidden;
   const float4 g0 = sum_runs4(partials, splits, t_count, n, t, r);
   const float4 g1 = sum_runs4(partials, splits, t_count, n, t, r + 4);
@@ -704,9 +774,8 @@ const char *rows_qkv_finish(const float *partials, int splits, int t, int q_head
                             float *v_cache, cudaStream_t stream) {
   if (hd % 8 != 0)
     return "the multi-position RoPE takes head_dim in multiples of 8";
-  const int64_t n = (int64_t)t * (q_heads + 2 * kv_heads) * (hd / 8);
-  launch_chained(qkv_finish_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0,
-                 stream, partials, splits, t, q_heads, kv_heads, hd, bias, cos_t,
+  const int n = (q_heads + 2 * kv_heads) * (hd / 8);
+  launch_chained(qkv_finish_kernel, dim3(t, (n + 255) / 256), dim3(256), 0, stream, partials, splits, t, q_heads, kv_heads, hd, bias, cos_t,
                  sin_t, first_pos, q_out, k_cache, v_cache);
   return last_launch("the multi-position RoPE and cache store");
 }
@@ -724,8 +793,13 @@ const char *rows_residual_norm(void *terms, float *x, const float *partials,
                                cudaStream_t stream) {
   if (dim > 256 * 32)
     return "the fused residual and RMSNorm take rows of at most 8192 values";
-  launch_chained(residual_norm_kernel, dim3(t), dim3(256), 0, stream,
-                 (__nv_bfloat16 *)terms, x, partials, splits, t, w, dim, eps);
+  const bool whole = dim % 4 == 0 && !(((uintptr_t)x | (uintptr_t)partials) & 15) &&
+                     !((uintptr_t)terms & 7);
+  auto kernel = !whole             ? residual_norm_kernel
+                : dim <= 4 * 4 * 256 ? residual_norm_quads_kernel<4>
+                                     : residual_norm_quads_kernel<8>;
+  launch_chained(kernel, dim3(t), dim3(256), 0, stream, (__nv_bfloat16 *)terms, x, partials,
+                 splits, t, w, dim, eps);
   return last_launch("the multi-position residual add and RMSNorm");
 }
 
@@ -733,10 +807,8 @@ const char *rows_swiglu_finish(void *terms, const float *partials, int splits, i
                                int hidden, cudaStream_t stream) {
   if (hidden % 8 != 0)
     return "the multi-position SwiGLU takes a hidden size in multiples of 8";
-  const int64_t count = (int64_t)t * (hidden / 8);
-  launch_chained(swiglu_finish_kernel, dim3((unsigned)((count + 255) / 256)),
-                 dim3(256), 0, stream, (__nv_bfloat16 *)terms, partials, splits, t,
-                 hidden);
+  launch_chained(swiglu_finish_kernel, dim3(t, (hidden / 8 + 255) / 256), dim3(256), 0, stream,
+                 (__nv_bfloat16 *)terms, partials, splits, t, hidden);
   return last_launch("the multi-position SwiGLU");
 }
 

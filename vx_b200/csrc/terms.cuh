@@ -40,6 +40,7 @@ namespace {
                                             int64_t t_count, int64_t n, int64_t t,
                                             int64_t r) {
   float4 s = *reinterpret_cast<const float4 *>(partials + t * n + r);
+#pragma unroll 4
   for (int k = 1; k < splits; ++k) {
     const float4 v = *reinterpret_cast<const float4 *>(
         partials + ((int64_t)k * t_count + t) * n + r);
