@@ -7,6 +7,7 @@ the vx_nn_* exports; flash_attention and gemm are the direct device-pointer
 calls of include/vx_b200.h.
 """
 import ctypes as C
+import functools
 
 import numpy as np
 
@@ -15,6 +16,7 @@ from .lib import check, lib
 
 
 # ---- a @ b --------------------------------------------------------------------
+@functools.lru_cache(maxsize=64)
 def _matmul_payload(name, outkind, topo, roles="a:0,b:1,out:2"):
     return abi.payload(name, abi=1, kind="matmul", roles=roles,
                        outkind=outkind, topo=topo)
@@ -23,6 +25,8 @@ def _matmul_payload(name, outkind, topo, roles="a:0,b:1,out:2"):
 def matmul_into(c, a, b, name="vx_npu_kernel_0"):
     """spawn on(GPU) { matmul_into(&mut c, &a, &b) }: the result buffer is an
     operand, filled in place (outkind=buffer). a, b, c: DeviceTensor."""
+    if len(a.shape) == len(b.shape) == len(c.shape) == 2:
+        return abi.dispatch_matrices(_matmul_payload(name, "buffer", c.topo), a, b, c)
     da = abi.descriptor(a.ptr, a.shape)
     db = abi.descriptor(b.ptr, b.shape)
     dc = abi.descriptor(c.ptr, c.shape)
