@@ -62,6 +62,41 @@ def test_f32_products_of_any_shape(m, n, k, off, pad):
     assert np.abs((got - want) / scale).max() <= 1e-6
 
 
+# edges of the 32 x 32 tiles, of the 8, 32 and 128 of K between sums, of the runs of 2, 4
+# and 8 blocks, rows off the 16- and 8-byte grids, and with more blocks than fit at once
+SMALL = [(1, 1, 1, 0, 0), (31, 33, 3, 1, 0), (32, 32, 128, 0, 0), (33, 65, 129, 0, 1),
+         (64, 31, 256, 2, 2), (257, 300, 190, 0, 0), (8, 40, 3001, 4, 4), (70, 96, 1023, 0, 0),
+         (200, 100, 512, 3, 1), (512, 512, 100, 0, 0)]
+
+
+@pytest.mark.parametrize("m,n,k,off,pad", SMALL)
+def test_f32_products_in_small_tiles(m, n, k, off, pad):
+    """A sum of four products, two of those, the exact sum of these sums and one last
+    rounding: six roundings of at most 2^-24 of the sum of magnitudes, and what the
+    rest's own sum loses, 2^-24 of 2^-24 of it for each eight of K."""
+    rng = np.random.default_rng(m * n + k)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = (rng.uniform(-1, 1, (k, n)) * 10.0 ** rng.uniform(-3, 3, (k, 1))).astype(np.float32)
+    got = product(a, b, m, n, k, abi.F32, offsets=(off, off, off), pads=(pad, pad, pad))
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    assert (np.abs(got - want) <= (6 + k / 8 * 2.0 ** -24) * 2.0 ** -24 * size).all()
+
+
+# the 128 x 128 tiles alone and in clusters of two, four and eight
+@pytest.mark.parametrize("m,n,k", [(1030, 520, 577), (1500, 1500, 130), (600, 600, 641),
+                                   (330, 300, 2500)])
+def test_f32_products_in_large_tiles(m, n, k):
+    rng = np.random.default_rng(k)
+    a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+    got = product(a, b, m, n, k, abi.F32)
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    scale = np.sqrt((a.astype(np.float64) ** 2).sum(1))[:, None] * \
+        np.sqrt((b.astype(np.float64) ** 2).sum(0))[None, :]
+    assert np.abs((got - want) / scale).max() <= 1e-6
+
+
 @pytest.mark.parametrize("k", [150, 1100])
 def test_f32_values_that_three_bf16_terms_cannot_carry(k):
     """Infinities, NaN, values whose terms' products would overflow, and values below the

@@ -28,7 +28,8 @@ SOURCES = ["rowdot_quant.cu", "rowdot_bf16.cu", "rowdot_f32.cu", "nn_kernels.cu"
            "dispatch.cu", "gemm_simt.cu", "gemm_umma.cu", "gemm_umma_pair.cu",
            "nn_api.cu", "decoder.cu", "decoder_parallel.cu", "flash_attn.cu",
            "static_scratch.cu", "rowdot_umma.cu", "prefill.cu", "prompt_attention.cu",
-           "quantize.cu", "step_kernel.cu", "gemm_f32_split.cu", "gemm_f32_tile.cu", "moe_group.cu",
+           "quantize.cu", "step_kernel.cu", "gemm_f32_split.cu", "gemm_f32_tile.cu", "gemm_f32_small.cu",
+           "moe_group.cu",
            "moe_grouped.cu", "q4_tiles.cu", "gemm_fp8_rows.cu", "window_attention.cu",
            "parallel_block.cu", "tensor_map.cu", "decoder_streams.cu",
            "latent_attention.cu", "gated_linear.cu", "residual_streams.cu",

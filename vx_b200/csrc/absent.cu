@@ -12,6 +12,8 @@ ABSENT(gemm_f32_split, const float *, int64_t, const float *, int64_t, float *, 
        int64_t, int64_t, int64_t, void *, Stream)
 ABSENT(gemm_f32_tile, const float *, int64_t, const float *, int64_t, float *, int64_t,
        int64_t, int64_t, int64_t, Stream)
+ABSENT(gemm_f32_small, const float *, int64_t, const float *, int64_t, float *, int64_t,
+       int64_t, int64_t, int64_t, Stream)
 ABSENT(gemm_f64, const double *, int64_t, const double *, int64_t, double *, int64_t,
        int64_t, int64_t, int64_t, Stream)
 ABSENT(gemm_16, bool, const void *, int64_t, const void *, int64_t, void *, int64_t,
@@ -47,6 +49,7 @@ size_t gemm_16_scratch_bytes(const void *, int64_t, const void *, int64_t, int64
                              int64_t) {
   return 0;
 }
+double gemm_f32_small_us(int64_t, int64_t, int64_t) { return 0.0; }
 double gemm_f32_tile_us(int64_t, int64_t, int64_t) { return 0.0; }
 double gemm_f32_split_us(int64_t, int64_t, int64_t, int64_t) { return 0.0; }
 size_t batched_proj_scratch_floats(int, int) { return 0; }

@@ -655,9 +655,11 @@ void gemm_on_device(const vx_gemm_plan &p, const Staged &a, const Staged &b,
   const char *why = nullptr;
   switch (p.dtype) {
   case VX_DTYPE_F32: {
-    /* on the tensor cores as exact bf16 terms (VXB_F32_TENSOR=0: always the FP32
-       pipe): the terms made inside the kernel, or beforehand for whole tiles of large
-       products, whichever takes less time */
+    /* on the FP32 pipe in small tiles, or on the tensor cores as exact bf16 terms
+       (VXB_F32_TENSOR=0: always the FP32 pipe, in large tiles): the terms made inside the
+       kernel, or beforehand for whole tiles of large products, whichever takes less time.
+       The first has to be 2.5 us ahead of the second: what the time model of the second
+       gives for its smallest products is more than that above what they take in a graph. */
     const char *off = getenv("VXB_F32_TENSOR");
     if (off && off[0] == '0') {
       why = vxb::gemm_f32((const float *)a.ptr, a.row_stride,
@@ -665,9 +667,14 @@ void gemm_on_device(const vx_gemm_plan &p, const Staged &a, const Staged &b,
                           p.m, p.n, p.k, t_stream);
       break;
     }
+    const double tile_us = vxb::gemm_f32_tile_us(p.m, p.n, p.k);
+    if (vxb::gemm_f32_small_us(p.m, p.n, p.k) + 2.5 < tile_us) {
+      why = vxb::gemm_f32_small((const float *)a.ptr, a.row_stride, (const float *)b.ptr,
+                                b.row_stride, (float *)c, ldc, p.m, p.n, p.k, t_stream);
+      break;
+    }
     const size_t need = vxb::gemm_f32_split_scratch_bytes(p.m, p.n, p.k, ldc);
-    if (need && vxb::gemm_f32_split_us(p.m, p.n, p.k, ldc) <
-                    vxb::gemm_f32_tile_us(p.m, p.n, p.k)) {
+    if (need && vxb::gemm_f32_split_us(p.m, p.n, p.k, ldc) < tile_us) {
       Staged scratch = Staged::temporary(need, 0, true);
       if (scratch.ptr) {
         why = vxb::gemm_f32_split((const float *)a.ptr, a.row_stride,

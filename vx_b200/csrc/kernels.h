@@ -29,7 +29,12 @@ const char *gemm_f32_split(const float *a, int64_t lda, const float *b, int64_t 
 const char *gemm_f32_tile(const float *a, int64_t lda, const float *b, int64_t ldb,
                           float *c, int64_t ldc, int64_t m, int64_t n, int64_t k,
                           cudaStream_t stream);
-/* What either takes, about, in microseconds. */
+/* The same on the FP32 pipe, for few tiles (gemm_f32_small.cu): any stride and alignment. */
+const char *gemm_f32_small(const float *a, int64_t lda, const float *b, int64_t ldb,
+                           float *c, int64_t ldc, int64_t m, int64_t n, int64_t k,
+                           cudaStream_t stream);
+/* What each takes, about, in microseconds. */
+double gemm_f32_small_us(int64_t m, int64_t n, int64_t k);
 double gemm_f32_tile_us(int64_t m, int64_t n, int64_t k);
 double gemm_f32_split_us(int64_t m, int64_t n, int64_t k, int64_t ldc);
 const char *gemm_f64(const double *a, int64_t lda, const double *b, int64_t ldb,
