@@ -368,6 +368,7 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
   ptx::tc_fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
+  chain_release();
 
   if (warp == 0) {
     /* ------------------------------------------------------------ loader */
@@ -375,6 +376,9 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
       ptx::tma_prefetch_desc(&map_q);
       ptx::tma_prefetch_desc(&map_k);
       ptx::tma_prefetch_desc(&map_v);
+      /* Set up under the tail of the kernel before: nothing is read before this, and
+         nothing written before what is read here has been multiplied. */
+      chain_wait();
       const int q_tiles = two ? NQ : 1;
       ptx::mbar_expect_tx(&bars->q_full, q_tiles * TILE_BYTES);
       for (int w = 0; w < q_tiles; ++w)
@@ -702,10 +706,10 @@ const char *flash_attention_fwd(const void *q, const void *k, const void *v,
   if (blocks > INT32_MAX)
     return "flash attention is asked for too many tiles";
   const dim3 grid((unsigned)blocks);
-  kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(
-      mq, mk, mv, (__nv_bfloat16 *)out, S, pairs, scale * 1.4426950408889634f,
-      causal ? 1 : 0);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      launch_chained(kernel, grid, dim3(THREADS), SMEM_BYTES, stream, mq, mk, mv,
+                     (__nv_bfloat16 *)out, S, pairs, scale * 1.4426950408889634f,
+                     causal ? 1 : 0);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 

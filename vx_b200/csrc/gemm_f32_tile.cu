@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tile_kernel(const TileGem
   ptx::tc_fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
+  chain_release();
+  chain_wait(); /* set up under the tail of the kernel before */
 
   /* the sums of a loader thread: row 32 (warp % 4) + lane of the tile, 32 columns */
   float acc[32];
@@ -459,19 +461,11 @@ const char *gemm_f32_tile(const float *a, int64_t lda, const float *b, int64_t l
   g.z = z;
   if (allow_dynamic_smem((const void *)gemm_f32_tile_kernel, SMEM_BYTES) != cudaSuccess)
     return "the f32 GEMM could not get its shared memory";
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((n + BN - 1) / BN * z), (unsigned)((m + BM - 1) / BM));
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)z;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = z > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel, g);
+  const dim3 grid((unsigned)((n + BN - 1) / BN * z), (unsigned)((m + BM - 1) / BM));
+  const cudaError_t e =
+      z > 1 ? launch_chained_cluster_smem(gemm_f32_tile_kernel, grid, dim3(THREADS), z,
+                                          SMEM_BYTES, stream, g)
+            : launch_chained(gemm_f32_tile_kernel, grid, dim3(THREADS), SMEM_BYTES, stream, g);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 

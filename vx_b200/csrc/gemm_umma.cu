@@ -154,12 +154,16 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   ptx::tc_fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
+  chain_release();
 
   if (warp == 0) {
     /* ---------------------------------------------------------- loader */
     if (lane == 0) {
       ptx::tma_prefetch_desc(&map_a);
       ptx::tma_prefetch_desc(&map_b);
+      /* Set up under the tail of the kernel before: nothing is read before this, and
+         nothing written before what is read here has been multiplied. */
+      chain_wait();
       int it = 0;
       bool ok = true;
       for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
@@ -379,7 +383,7 @@ const char *launch_umma(const CUtensorMap &ma, const CUtensorMap &mb, const Out<
   const int64_t items =
       (int64_t)((m + BM - 1) / BM) * ((n + BN - 1) / BN) * out.runs;
   const int grid = (int)(items < sm_count() ? items : sm_count());
-  kernel<<<grid, THREADS, bytes, stream>>>(ma, mb, out, m, n, k);
+  launch_chained(kernel, dim3(grid), dim3(THREADS), bytes, stream, ma, mb, out, m, n, k);
   if (out.runs > 1)
     launch_chained(finish16_kernel<T>,
                    dim3((unsigned)(((int64_t)m * out.pitch + 255) / 256)), dim3(256), 0,

@@ -121,12 +121,16 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   ptx::tc_fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
+  chain_release();
 
   if (warp == 0) {
     /* ---------------------------------------------------------- loader */
     if (lane == 0) {
       ptx::tma_prefetch_desc(&map_a);
       ptx::tma_prefetch_desc(&map_b);
+      /* Set up under the tail of the kernel before: nothing is read before this, and
+         nothing written before what is read here has been multiplied. */
+      chain_wait();
       int it = 0;
       bool ok = true;
       for (int tile = pair; ok && tile < tiles; tile += pairs) {
@@ -304,10 +308,10 @@ const char *launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, void *c,
   }
   if (pairs > tiles)
     pairs = tiles;
-  cfg.gridDim = dim3(2 * pairs);
   const int vec = ((uintptr_t)c & 15) == 0 && ldc % 8 == 0;
-  const cudaError_t e =
-      cudaLaunchKernelEx(&cfg, kernel, ma, mb, (T *)c, ldc, m, n, k, vec);
+  const cudaError_t e = launch_chained_cluster_smem(kernel, dim3(2 * pairs), dim3(THREADS), 2,
+                                                    SMEM_BYTES, stream, ma, mb, (T *)c, ldc, m,
+                                                    n, k, vec);
   return e == cudaSuccess ? nullptr : cudaGetErrorString(e);
 }
 
