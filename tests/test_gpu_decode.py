@@ -112,6 +112,31 @@ def test_nn_decoder_keeps_every_device_table_it_reads(oracle):
     assert got == want, report(got, want)
 
 
+def test_more_decoders_at_once_than_have_room_in_the_pinned_page(oracle):
+    """34 decoders, of which 32 leave their tokens where the host reads them and two are
+    copied; rooms given back are used again; none may see another's token."""
+    flat, offsets = llama.small_f32_weights()
+    cfg = oracle.LlamaConfig(288, 768, 6, 6, 6, 32000, 256)
+    want = {t: list(oracle.llama_generate(cfg, flat, t, 4)) for t in (1, 17, 31999)}
+    first = [(1, 17, 31999)[i % 3] for i in range(34)]
+    decs = [llama.small_f32_decoder(flat, offsets) for _ in first]
+    got = [[t] for t in first]
+    for step in range(3):
+        for d, t, out in zip(decs, first, got):
+            out.append(d.step([t] if step == 0 else None)[0])
+    for i in (0, 31, 33):
+        decs[i].close()
+        decs[i] = llama.small_f32_decoder(flat, offsets)
+        got[i] = [first[i]]
+    for i, d in enumerate(decs):
+        while len(got[i]) < 5:
+            got[i].append(d.step([first[i]] if len(got[i]) == 1 else None)[0])
+    for d in decs:
+        d.close()
+    for t, out in zip(first, got):
+        assert out == want[t][:5], report(out, want[t])
+
+
 @pytest.mark.parametrize("q_heads,kv_heads", [(4, 4), (4, 2), (8, 2)])
 def test_one_launch_step_matches_the_oracle_and_the_separate_kernels(
         oracle, monkeypatch, q_heads, kv_heads):

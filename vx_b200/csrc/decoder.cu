@@ -39,6 +39,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <utility>
 #include <string>
 #include <vector>
@@ -339,19 +340,21 @@ void decoder_record_tail(vx_decoder *d, int launches) {
   const int B = c.batch;
   cudaStream_t s = d->stream;
   if (d->ranks == 1) {
-    need(vxb::argmax(d->tokens, d->logits, d->vocab_local, B, d->logit_stride, s),
+    need(vxb::argmax(d->tokens, d->logits, d->vocab_local, B, d->logit_stride, s, d->told,
+                     d->positions),
          "argmax");
-    launches += 1;
+    d->kernels_per_step = launches + 1;
+    return;
+  }
+  need(vxb::argmax(d->local_best, d->logits, d->vocab_local, B,
+                   d->vocab_local, s),
+       "argmax");
+  if (d->push) {
+    tp_pick_kernel<<<1, d->ranks * 32, 0, s>>>(
+        d->tokens, d->local_best, d->logits, d->vocab_local, d->vocab_offset,
+        d->pick, d->ranks, d->tp.rank, B, d->pick_epoch, d->pick_gave_up);
+    launches += 2;
   } else {
-    need(vxb::argmax(d->local_best, d->logits, d->vocab_local, B,
-                     d->vocab_local, s),
-         "argmax");
-    if (d->push) {
-      tp_pick_kernel<<<1, d->ranks * 32, 0, s>>>(
-          d->tokens, d->local_best, d->logits, d->vocab_local, d->vocab_offset,
-          d->pick, d->ranks, d->tp.rank, B, d->pick_epoch, d->pick_gave_up);
-      launches += 2;
-    } else {
     best_pair_kernel<<<1, B, 0, s>>>(d->pair, d->local_best, d->logits,
                                      d->vocab_local, d->vocab_offset);
     vx::NcclCollective *job = vxb::nccl_job();
@@ -362,7 +365,6 @@ void decoder_record_tail(vx_decoder *d, int launches) {
            job->api()->GetErrorString(r));
     pick_pair_kernel<<<1, 32, 0, s>>>(d->tokens, d->pairs_all, d->ranks, B);
     launches += 4;
-    }
   }
   advance_kernel<<<1, 32, 0, s>>>(d->positions, B);
   ++launches;
@@ -631,6 +633,34 @@ void record_step(vx_decoder *d, int max_pos) {
   decoder_record_tail(d, launches);
 }
 
+/* One page of pinned memory a process, in which each decoder has room for its 32 tokens;
+   NULL for a decoder beyond the 32nd at a time, whose tokens are copied. (To allocate and
+   free one for each decoder takes milliseconds.) */
+std::mutex g_told_mu;
+int32_t *g_told = nullptr;
+uint32_t g_told_taken = 0;
+int32_t *take_told() {
+  std::lock_guard<std::mutex> lock(g_told_mu);
+  if (!g_told && cudaHostAlloc((void **)&g_told, 32 * 32 * sizeof(int32_t),
+                               cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    g_told = nullptr;
+    return nullptr;
+  }
+  for (int i = 0; i < 32; ++i)
+    if (!(g_told_taken >> i & 1)) {
+      g_told_taken |= 1u << i;
+      return g_told + 32 * i;
+    }
+  return nullptr;
+}
+void give_told(int32_t *told) {
+  if (!told)
+    return;
+  std::lock_guard<std::mutex> lock(g_told_mu);
+  g_told_taken &= ~(1u << ((told - g_told) / 32));
+}
+
 cudaGraphExec_t graph_for(vx_decoder *d, int bucket) {
   auto hit = d->graphs.find(bucket);
   if (hit != d->graphs.end())
@@ -848,6 +878,7 @@ void vx_decoder_destroy(vx_decoder *d) {
   decoder_free_parallel(d);
   decoder_free_streams(d);
   cudaFree(d->owned_weights);
+  give_told(d->told);
   cudaStreamDestroy(d->stream);
   delete d;
 }
@@ -876,6 +907,8 @@ int32_t vx_decoder_step(vx_decoder *d, const int32_t *tokens_in,
   const int pos = d->host_pos;
   if (pos >= d->c.max_seq)
     stop("vx_decoder_step: position %d is past max_seq %d", pos, d->c.max_seq);
+  if (d->ranks == 1 && !d->told && d->graphs.empty())
+    d->told = take_told();
   cudaGraphExec_t exec = graph_for(d, d->one_kernel || d->par || d->streams ? 0 : pos / 256);
   if (tokens_in)
     CUDA_OK(cudaMemcpyAsync(d->tokens, tokens_in, d->c.batch * sizeof(int32_t),
@@ -883,11 +916,14 @@ int32_t vx_decoder_step(vx_decoder *d, const int32_t *tokens_in,
   CUDA_OK(cudaGraphLaunch(exec, d->stream));
   d->host_pos = pos + 1;
   if (tokens_out) {
-    CUDA_OK(cudaMemcpyAsync(tokens_out, d->tokens, d->c.batch * sizeof(int32_t),
-                            cudaMemcpyDeviceToHost, d->stream));
+    if (!d->told)
+      CUDA_OK(cudaMemcpyAsync(tokens_out, d->tokens, d->c.batch * sizeof(int32_t),
+                              cudaMemcpyDeviceToHost, d->stream));
     const cudaError_t e = cudaStreamSynchronize(d->stream);
     if (e != cudaSuccess)
       stop("a kernel of the decoder faulted: %s", cudaGetErrorString(e));
+    if (d->told)
+      memcpy(tokens_out, d->told, d->c.batch * sizeof(int32_t));
   }
   return pos;
 }

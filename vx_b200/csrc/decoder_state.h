@@ -139,6 +139,8 @@ struct vx_decoder {
   float *x, *xn, *q, *att, *h, *tmp, *logits, *k_cache, *v_cache, *scratch;
   bool fused_norm; /* the activations of all sequences fit the projections' shared memory */
   int32_t *tokens, *positions, *counters, *local_best;
+  /* the tokens of a step once more, in pinned memory (one rank) */
+  int32_t *told = nullptr;
   float2 *pair, *pairs_all;
   /* tp_reduce == 1: partial sums exchanged through peer memory */
   bool push;

@@ -421,7 +421,8 @@ int blocks_of_tile(int64_t m, int64_t n, int64_t k) {
    memory and 176 KiB read from it, and sixteen warps splitting) and 7.4 for a tile's start
    and end, as many rounds as the tiles need. Measured 24.6 / 51.4 / 126 / 365 / 65.6 / 38.8
    at 1024^3, 1536^3, 2048^3, 3072^3, 2944 x 2944 x 320, 128 x 128 x 8192, where this gives
-   24.6 / 51.8 / 127 / 360 / 67 / 38.2. */
+   24.6 / 51.8 / 127 / 360 / 67 / 38.2. (A call by itself, of which 3.4 go under the tail
+   of the call before where there is one.) */
 double gemm_f32_tile_us(int64_t m, int64_t n, int64_t k) {
   if ((m + BM - 1) / BM > kMostRowTiles)
     return HUGE_VAL;

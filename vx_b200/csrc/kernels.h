@@ -743,7 +743,8 @@ const char *moe_down_q4_add_grouped(const MoeGroupedArgs &m, cudaStream_t stream
    pair outside `order`); waits for the stream. */
 int moe_group_status(cudaStream_t stream);
 const char *argmax(int32_t *out, const float *logits, int n, int batch,
-                   int64_t stride, cudaStream_t stream);
+                   int64_t stride, cudaStream_t stream, int32_t *host = nullptr,
+                   int32_t *positions = nullptr);
 const char *embed(float *x, const void *table, bool tbf16, const int32_t *token,
                   int dim, int rows, int batch, int64_t x_stride,
                   cudaStream_t stream);
