@@ -533,6 +533,7 @@ void record_step(vx_decoder *d, int max_pos) {
     qa.v_cache = d->v_cache + l * d->cache_layer_stride;
     qa.cache_batch_stride = d->cache_batch_stride;
     qa.max_seq = c.max_seq;
+    qa.weights_settled = 1; /* older than the graph */
     need(vxb::qkv_rope_store(qa, s), "q/k/v");
 
     vxb::AttnArgs aa{};
@@ -567,6 +568,7 @@ void record_step(vx_decoder *d, int max_pos) {
     oa.y_stride = c.dim;
     oa.mode = d->push ? 3 : (d->ranks > 1 ? 0 : 1);
     oa.push = &d->tp;
+    oa.weights_settled = 1;
     need(vxb::matvec(oa, s), "the output projection");
     launches += 3;
     launches += add_partials(d);
@@ -587,6 +589,7 @@ void record_step(vx_decoder *d, int max_pos) {
     sa.norm_w = d->fused_norm ? d->ffn_norm[l] : nullptr;
     sa.norm_bf16 = bf;
     sa.eps = c.eps;
+    sa.weights_settled = 1;
     need(vxb::swiglu(sa, s), "gate/up");
 
     vxb::MatvecArgs da{};
@@ -603,6 +606,7 @@ void record_step(vx_decoder *d, int max_pos) {
     da.y_stride = c.dim;
     da.mode = d->push ? 3 : (d->ranks > 1 ? 0 : 1);
     da.push = &d->tp;
+    da.weights_settled = 1;
     need(vxb::matvec(da, s), "the down projection");
     launches += 2;
     launches += add_partials(d);
@@ -627,6 +631,7 @@ void record_step(vx_decoder *d, int max_pos) {
   la.y = d->logits;
   la.y_stride = d->vocab_local;
   la.mode = 0;
+  la.weights_settled = 1;
   need(vxb::matvec(la, s), "the logits");
   ++launches;
   }

@@ -183,6 +183,7 @@ void decoder_record_parallel_step(vx_decoder *d) {
     o.y = d->x;
     o.y_stride = c.dim;
     o.mode = 1;
+    o.weights_settled = 1;
     need(vxb::matvec(o, s), "the output projection");
     launches += 3;
   }
@@ -200,6 +201,7 @@ void decoder_record_parallel_step(vx_decoder *d) {
   h.y = d->logits;
   h.y_stride = p.vocab_rows;
   h.mode = 0;
+  h.weights_settled = 1;
   need(vxb::matvec(h, s), "the logits");
   decoder_record_tail(d, launches + 1);
 }

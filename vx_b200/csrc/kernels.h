@@ -102,6 +102,13 @@ struct MatvecArgs {
                           3 y += the sum of all ranks' s (see TpPush) */
   const void *bias;    /* mode 2, bf16 */
   const struct TpPush *push; /* mode 3 */
+  /* 1: the caller vouches that w and scales were written before the chain of dependent
+     launches this kernel is part of began (a decoder's are older than its graph), or that
+     the kernel in front has waited for whatever wrote them: they are fetched before the
+     wait for it. 0: everything is read after that wait. A call whose matrix the kernel in
+     front may just have made (a product, say, which lets its successor start while it
+     still stores) leaves it 0. */
+  int weights_settled;
 };
 
 /* Mode 3: the projection is one rank's partial of a row-split product, and
@@ -153,6 +160,7 @@ struct SwigluArgs {
   const void *norm_w;
   bool norm_bf16;
   float eps;
+  int weights_settled; /* as in MatvecArgs */
 };
 const char *swiglu(const SwigluArgs &a, cudaStream_t stream);
 
@@ -187,6 +195,7 @@ struct QkvArgs {
   float *k_cache, *v_cache;
   int64_t cache_batch_stride;
   int max_seq;
+  int weights_settled; /* as in MatvecArgs */
 };
 const char *qkv_rope_store(const QkvArgs &a, cudaStream_t stream);
 
@@ -196,7 +205,9 @@ const char *qkv_rope_store(const QkvArgs &a, cudaStream_t stream);
  *   q | k | gate | up,
  * in that order, and its results go four ways: q as they are; k into row
  * position % cache_rows of a ring of keys; sigmoid(gate); relu(up)^2. The
- * output matrix has the columns of the attention output, then those of `up`. */
+ * output matrix has the columns of the attention output, then those of `up`.
+ * The weights of fan_proj, and of stream_proj below, are a decoder's: settled, as
+ * MatvecArgs has it. */
 struct FanOut {
   int k_row, gate_row, up_row; /* where each part begins; multiples of 8 */
   int cache_rows;
@@ -362,6 +373,7 @@ const char *attention_decode_clustered(const AttnArgs &a, cudaStream_t stream);
  * terms (rowdot_umma.cu). mode: 0 y = s, 1 y += s, 3 SwiGLU (rows = units; w0
  * gate rows, w1 up rows or NULL: up rows follow in w0), 4 q/k/v + bias + RoPE +
  * KV store (head_dim 128; w1/w2 k and v matrices or NULL: rows follow in w0).
+ * The weights are a decoder's: settled, as MatvecArgs has it.
  * xs: bf16 [48 or 32][cols] work space for the terms; scratch:
  * batched_proj_scratch_floats() floats for the partial sums of the K runs. */
 struct BatchedProj {

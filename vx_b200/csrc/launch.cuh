@@ -8,7 +8,10 @@
  * not depend on N (for a projection: filling their shared-memory ring with
  * weights), and only then wait for N (griddepcontrol.wait).  Every kernel
  * launched through launch_chained() calls chain_wait() before it touches
- * anything an earlier kernel wrote.
+ * anything an earlier kernel of its chain wrote.  What a kernel may fetch before
+ * that, weights and rows of a cache, its caller has said to be older than the chain
+ * (weights_settled and rows_settled in kernels.h): a kernel releases its successor
+ * before it has stored anything.
  *
  * VXB_PDL=0 in the environment turns the attribute off (plain stream order).
  */

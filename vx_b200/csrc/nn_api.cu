@@ -259,6 +259,7 @@ void vx_nn_qkv(VX_TENSOR2(q), VX_TENSOR2(k), VX_TENSOR2(v), VX_TENSOR1(w),
     a.batch = 1;
     a.mode = 2;
     a.bias = bp + row;
+    a.weights_settled = part > 0; /* part 0 has waited for what made them */
     must(vxb::matvec(a, vxb::caller_stream()), FN);
     row += a.rows;
   }
@@ -420,7 +421,7 @@ void check_quant(const char *fn, int quant, int64_t w_len, int64_t s_len,
 void quant_matvec(const char *fn, int quant, float *y, int64_t y_len,
                   const void *w, int64_t w_len, const void *scales,
                   int64_t s_len, const float *x, int64_t x_len, int rows,
-                  int cols, int mode) {
+                  int cols, int mode, bool settled = false) {
   check_quant(fn, quant, w_len, s_len, x_len, rows, cols);
   if (y_len < rows)
     stop("%s: the output has fewer values than rows", fn);
@@ -436,12 +437,14 @@ void quant_matvec(const char *fn, int quant, float *y, int64_t y_len,
   a.y_stride = rows;
   a.batch = 1;
   a.mode = mode;
+  a.weights_settled = settled;
   must(vxb::matvec(a, vxb::caller_stream()), fn);
 }
 void quant_qkv(const char *fn, int quant, float *q, float *k, float *v,
                const void *w, int64_t w_len, const void *scales, int64_t s_len,
                const uint16_t *bias, int64_t b_len, const float *x,
-               int64_t x_len, int q_heads, int kv_heads, int head_dim, int cols) {
+               int64_t x_len, int q_heads, int kv_heads, int head_dim, int cols,
+               bool settled = false) {
   const int rows_all = (q_heads + 2 * kv_heads) * head_dim;
   check_quant(fn, quant, w_len, s_len, x_len, rows_all, cols);
   if (b_len < rows_all)
@@ -465,6 +468,7 @@ void quant_qkv(const char *fn, int quant, float *q, float *k, float *v,
     a.batch = 1;
     a.mode = 2;
     a.bias = bias + row;
+    a.weights_settled = settled || part > 0; /* part 0 has waited for what made them */
     must(vxb::matvec(a, vxb::caller_stream()), fn);
     row += a.rows;
   }
@@ -734,6 +738,7 @@ void vx_nn_matvec_rows(VX_TENSOR2(y), VX_TENSOR1(w), VX_TENSOR2(x), int32_t n,
     a.y_stride = y_n1;
     a.batch = chunk;
     a.mode = 0;
+    a.weights_settled = t > 0; /* the first chunk has waited for what made them */
     must(vxb::matvec(a, vxb::caller_stream()), FN);
   });
 }
@@ -749,7 +754,7 @@ void vx_nn_matvec_q4_rows(VX_TENSOR2(y), VX_TENSOR1(w), VX_TENSOR1(scales),
   for (int t = 0; t < n; ++t)
     quant_matvec(FN, vxb::kFmtQ4, yp + (int64_t)t * y_n1, y_n1, T1(uint32_t, w),
                  w_n0, T1(uint16_t, scales), scales_n0, xp + (int64_t)t * x_n1,
-                 x_n1, rows, cols, 0);
+                 x_n1, rows, cols, 0, t > 0);
 }
 #undef FN
 
@@ -832,7 +837,7 @@ void vx_nn_matvec_q4_heads_add_rows(VX_TENSOR2(y), VX_TENSOR1(w), VX_TENSOR1(sca
     quant_matvec(FN, vxb::kFmtQ4, yp + (int64_t)t * y_n1, y_n1, T1(uint32_t, w),
                  w_n0, T1(uint16_t, scales), scales_n0,
                  xp + (int64_t)t * x_n1 * x_n2, (int64_t)heads * head_dim, rows,
-                 heads * head_dim, 1);
+                 heads * head_dim, 1, t > 0);
 }
 #undef FN
 
@@ -855,7 +860,7 @@ void vx_nn_qkv_q4_rows(VX_TENSOR3(q), VX_TENSOR3(k), VX_TENSOR3(v), VX_TENSOR1(w
               kp + (int64_t)t * k_n1 * k_n2, vp + (int64_t)t * v_n1 * v_n2,
               T1(uint32_t, w), w_n0, T1(uint16_t, scales), scales_n0,
               T1(uint16_t, b), b_n0, xp + (int64_t)t * x_n1, x_n1, q_heads,
-              kv_heads, head_dim, cols);
+              kv_heads, head_dim, cols, t > 0);
 }
 #undef FN
 

@@ -476,15 +476,20 @@ __host__ __device__ constexpr bool reads_streams(int epi) {
 }
 
 struct RowDotParams {
-  /* weights */
-  const void *w0, *w1, *w2; /* matvec: w0; swiglu: gate w0, up w1; qkv: q,k,v */
+  /* What a kernel needs before its first copies lies together: each line of the
+     parameters that it touches is a trip to memory of its own. */
+  const void *w0, *w1; /* matvec: w0; swiglu: gate w0, up w1; qkv: q, k (v: w2) */
+  const void *s0, *s1; /* their scales, see s2 */
+  const int32_t *expert_ids; /* see expert_slot */
+  int rows, cols;
+  int items;
+  int weights_settled; /* see MatvecArgs in kernels.h */
+  int row_base;        /* see s2 */
+  const void *w2;
   /* the scales of w0, w1, w2 (fp8: f32 [ceil(rows/128), cols/128]; Q4_0: f16
      [rows, cols/32]); row_base: the row of the whole matrix that row 0 of w0
      is, when w0 is a run of rows inside a matrix with one table of scales */
-  const void *s0, *s1, *s2;
-  int row_base;
-  int rows, cols;
-  int items;
+  const void *s2;
   /* activations */
   const float *x;
   int64_t x_stride;
@@ -512,7 +517,6 @@ struct RowDotParams {
      another, expert_bytes (scale_bytes) apart, and this launch takes matrix
      expert_ids[expert_slot] (device memory: the router wrote it). add_scale
      (EPI_ADD): y += add_scale[0] * s. */
-  const int32_t *expert_ids;
   int expert_slot, experts;
   int64_t expert_bytes, scale_bytes;
   const float *add_scale;

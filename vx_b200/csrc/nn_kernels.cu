@@ -337,6 +337,7 @@ const char *matvec(const MatvecArgs &a, cudaStream_t stream) {
   p.bias = a.bias;
   p.s0 = a.scales;
   p.row_base = a.row_base;
+  p.weights_settled = a.weights_settled;
   const int fmt = a.wfmt ? a.wfmt : (a.wbf16 ? kFmtBf16 : kFmtF32);
   const int per_word = fmt == kFmtF32 ? 4 : fmt == kFmtBf16 ? 8 : fmt == kFmtFp8 ? 16 : 32;
   if (a.expert_ids) {
@@ -405,6 +406,7 @@ const char *fan_proj(const FanArgs &a, cudaStream_t stream) {
   p.cache_batch_stride = a.cache_batch_stride;
   p.positions = a.positions;
   p.fan = a.out;
+  p.weights_settled = 1;
   return launch_rowdot(EPI_FAN, p, a.fmt, stream);
 }
 
@@ -434,6 +436,7 @@ const char *stream_proj(const StreamProj &a, cudaStream_t stream) {
   p.stream_out = a.out;
   p.logit_scale = a.logit_scale;
   p.logit_cap = a.logit_cap;
+  p.weights_settled = 1;
   switch (a.mode) {
   case kStreamsStore: return launch_rowdot(EPI_IN_STORE, p, a.fmt, stream);
   case kStreamsGelu: return launch_rowdot(EPI_IN_GELU, p, a.fmt, stream);
@@ -466,6 +469,7 @@ const char *swiglu(const SwigluArgs &a, cudaStream_t stream) {
   p.s0 = a.scales;
   p.s1 = a.scales_up;
   p.row_base = a.row_base;
+  p.weights_settled = a.weights_settled;
   if (a.expert_ids) {
     const int fmt = a.wfmt ? a.wfmt : (a.wbf16 ? kFmtBf16 : kFmtF32);
     const int per_word = fmt == kFmtF32 ? 4 : fmt == kFmtBf16 ? 8 : fmt == kFmtFp8 ? 16 : 32;
@@ -514,6 +518,7 @@ const char *qkv_rope_store(const QkvArgs &a, cudaStream_t stream) {
   p.v_cache = a.v_cache;
   p.cache_batch_stride = a.cache_batch_stride;
   p.max_seq = a.max_seq;
+  p.weights_settled = a.weights_settled;
   p.s0 = a.sq;
   p.s1 = a.sk;
   p.s2 = a.sv;

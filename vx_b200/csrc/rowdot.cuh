@@ -308,7 +308,17 @@ rowdot_kernel(const RowDotParams p) {
       }
     }
   };
-  /* The weights do not depend on the kernel before this one: start them. */
+  /* Settled weights do not depend on the kernel before this one: start them. Of others
+     the first rows may come as far as L2, where whatever that kernel stores arrives too
+     (22016 x 4096 in bf16, one after another, us: 29.9 without, 28.9 with, 28.0 settled). */
+  if (!p.weights_settled) {
+    if (lane == 0 && units > 0) {
+      const int bytes = row_bytes < RING_STAGES * CHUNK_BYTES ? row_bytes : RING_STAGES * CHUNK_BYTES;
+      ptx::bulk_prefetch_l2(ld_r0, bytes);
+      ptx::bulk_prefetch_l2(ld_r1, bytes);
+    }
+    chain_wait();
+  }
   for (int u = 0; u < RING_STAGES; ++u)
     issue_next();
   chain_release();

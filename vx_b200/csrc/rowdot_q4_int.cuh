@@ -216,7 +216,9 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
     ld_tile = tiles;
   else if (ld_tile < tiles)
     open_tile();
-  /* The weights do not depend on the kernel before this one: start them. */
+  /* Settled weights do not depend on the kernel before this one: start them. */
+  if (!p.weights_settled)
+    chain_wait();
   for (int s = 0; s < STAGES; ++s)
     issue_next();
   chain_release();

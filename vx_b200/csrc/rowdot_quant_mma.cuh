@@ -255,7 +255,9 @@ quant_mma_kernel(const RowDotParams p, const QuantPlan plan,
     ++ld_ks;
     ld_stage = ld_stage + 1 == stages ? 0 : ld_stage + 1;
   };
-  /* The weights do not depend on the kernel before this one: start them. */
+  /* Settled weights do not depend on the kernel before this one: start them. */
+  if (!p.weights_settled)
+    chain_wait();
   if (gw < units) {
     open_unit(gw);
     for (int s = 0; s < stages; ++s)
