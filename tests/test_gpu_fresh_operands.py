@@ -93,3 +93,44 @@ def test_a_projection_reads_what_the_product_before_it_has_made(consumer, m, n, 
     assert ops.kernel_status() == 0
     for i in range(times):
         assert torch.equal(y[i], want[i % 2]), i
+
+
+@pytest.mark.parametrize("second", ["one CTA", "pairs", "attention"])
+def test_a_kernel_whose_predecessor_takes_longer_than_its_waits(second):
+    """The scalar product of two vectors of 4.8 GB is one small tile, a cluster of eight
+    blocks that take two seconds. What follows is set up on the other SMs meanwhile, and its
+    bounded waits, of about a second, must not have begun."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    long = 1_200_000_000
+    a, b = torch.full((1, long), 0.5, device="cuda"), torch.full((long, 1), 2.0, device="cuda")
+    c = torch.zeros((1, 1), device="cuda")
+
+    def rand(*shape):
+        return (torch.rand(shape, generator=g, device="cuda") - 0.5).bfloat16()
+    if second == "attention":
+        q, k, v = (rand(1, 2, 512, 128) for _ in range(3))
+        out, want = torch.zeros_like(q), torch.zeros_like(q)
+    else:
+        n = 384 if second == "one CTA" else 4096
+        q, k = rand(n, n), rand(n, n)
+        out, want = torch.zeros_like(q), torch.zeros_like(q)
+
+    def run(to):
+        if second == "attention":
+            ops.flash_attention(tensor(q), tensor(k), tensor(v), tensor(to), 128 ** -0.5, True)
+        else:
+            ops.matmul_into(tensor(to), tensor(q), tensor(k))
+    run(want)
+    torch.cuda.synchronize()
+    began, ended = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    began.record()
+    ops.matmul_into(tensor(c), tensor(a), tensor(b))
+    run(out)
+    ended.record()
+    torch.cuda.synchronize()
+    assert ops.kernel_status() == 0
+    assert began.elapsed_time(ended) > 1200     # else this shows nothing
+    assert torch.equal(out, want)
+    assert c.item() == long

@@ -370,6 +370,9 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
   chain_release();
+  /* Set up under the tail of the kernel before. Every warp waits for its end: the limits of
+     the waits below are for this kernel's own work. */
+  chain_wait();
 
   if (warp == 0) {
     /* ------------------------------------------------------------ loader */
@@ -377,9 +380,6 @@ flash_kernel(const __grid_constant__ CUtensorMap map_q,
       ptx::tma_prefetch_desc(&map_q);
       ptx::tma_prefetch_desc(&map_k);
       ptx::tma_prefetch_desc(&map_v);
-      /* Set up under the tail of the kernel before: nothing is read before this, and
-         nothing written before what is read here has been multiplied. */
-      chain_wait();
       const int q_tiles = two ? NQ : 1;
       ptx::mbar_expect_tx(&bars->q_full, q_tiles * TILE_BYTES);
       for (int w = 0; w < q_tiles; ++w)

@@ -155,15 +155,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
   chain_release();
+  /* Set up under the tail of the kernel before. Every warp waits for its end: the limits of
+     the waits below are for this kernel's own work. */
+  chain_wait();
 
   if (warp == 0) {
     /* ---------------------------------------------------------- loader */
     if (lane == 0) {
       ptx::tma_prefetch_desc(&map_a);
       ptx::tma_prefetch_desc(&map_b);
-      /* Set up under the tail of the kernel before: nothing is read before this, and
-         nothing written before what is read here has been multiplied. */
-      chain_wait();
       int it = 0;
       bool ok = true;
       for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {

@@ -248,7 +248,9 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
       }
     }
   } else if (warp == 1) {
-    /* ------------------------------------------------------ MMA issuer */
+    /* ------------------------------------------------------ MMA issuer
+       (whose waits, as the epilogue's, have limits for this kernel's own work) */
+    chain_wait();
     {
       const uint32_t idesc = ptx::idesc_f16(true, false, false, TM, p.n);
       int it = 0, t = 0;
@@ -293,6 +295,7 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
   } else {
     /* ---------------------------------------------------------- epilogue
        Four warps, a weight row per thread. */
+    chain_wait();
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane; /* row within the tile */
     const int B = p.batch;
