@@ -142,7 +142,6 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
   Bars *bars = reinterpret_cast<Bars *>(smem + STAGES * stage_bytes);
 
   const int warp = ptx::warp_index(), lane = threadIdx.x % 32;
-  chain_release();
   const int items = p.tiles * p.splits;
   /* item -> (tile, run of K blocks): runs of a tile are consecutive items */
   auto item_range = [&](int item, int &tile, int &split, int &kb0, int &kb1) {
@@ -172,6 +171,10 @@ rowdot_mma_kernel(const __grid_constant__ CUtensorMap map_w0,
   ptx::tc_fence_after_sync();
   const uint32_t tmem = bars->tmem_base;
   volatile int *stop = &bars->stop;
+  /* Not before the tensor memory is this block's: there is no limit to the wait for it, and
+     the kernel after the next, which starts once that one has released it, may want
+     columns too while it waits for this kernel's end. */
+  chain_release();
 
   if (warp == 0) {
     /* ---------------------------------------------------------- loader */
