@@ -413,6 +413,40 @@ def test_quantised_decoder_tokens_match_oracle(oracle, quant):
     assert got == want, report(got, want)
 
 
+@pytest.mark.parametrize("quant", ["fp8", "q4"])
+def test_quantised_decoder_with_gains_on_an_8_byte_boundary(quant, monkeypatch):
+    """The norms' gains as a slice of a larger tensor: the same logits, bit for bit."""
+    import torch
+    made = llama.Decoder
+
+    def moved(by):
+        def decoder(cfg, weights, keep=None):
+            g = torch.Generator(device="cuda")
+            g.manual_seed(1)
+            n, held = cfg.dim, []
+
+            def gains(_):
+                t = torch.zeros(n + 8, dtype=torch.bfloat16, device="cuda")
+                t[by:by + n] = 1 + 0.1 * torch.randn(n, generator=g, device="cuda")
+                held.append(t)
+                return t[by:].data_ptr()
+            weights = dict(weights, attn_norm=[gains(p) for p in weights["attn_norm"]],
+                           ffn_norm=[gains(p) for p in weights["ffn_norm"]],
+                           final_norm=gains(weights["final_norm"]))
+            torch.cuda.synchronize()
+            return made(cfg, weights, keep=(keep, held))
+        return decoder
+    logits = []
+    for by in (0, 4):
+        monkeypatch.setattr(llama, "Decoder", moved(by))
+        dec, _ = llama.nn_quant_model(quant, max_seq=32, **QUANT_NN)
+        for t in (5, 4000, 17):
+            dec.step([t])
+        logits.append(dec.logits())
+        dec.close()
+    assert np.isfinite(logits[0]).all() and np.array_equal(*logits)
+
+
 @pytest.mark.parametrize("quant,route", [("q4", ""), ("q4", "mma"), ("fp8", ""),
                                          ("fp8", "mma")])
 def test_prefill_with_quantised_weights(oracle, quant, route, monkeypatch):

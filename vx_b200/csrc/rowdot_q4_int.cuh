@@ -245,9 +245,11 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
         continue;
       float *w = ws[k];
       if (p.norm_bf16) {
-        const uint4 b = *reinterpret_cast<const uint4 *>((const uint16_t *)p.norm_w + c);
-        w[0] = bf_lo(b.x); w[1] = bf_hi(b.x); w[2] = bf_lo(b.y); w[3] = bf_hi(b.y);
-        w[4] = bf_lo(b.z); w[5] = bf_hi(b.z); w[6] = bf_lo(b.w); w[7] = bf_hi(b.w);
+        /* (gains on an 8-byte boundary, as the other projection kernels take them) */
+        const uint2 *b2 = reinterpret_cast<const uint2 *>((const uint16_t *)p.norm_w + c);
+        const uint2 a = b2[0], b = b2[1];
+        w[0] = bf_lo(a.x); w[1] = bf_hi(a.x); w[2] = bf_lo(a.y); w[3] = bf_hi(a.y);
+        w[4] = bf_lo(b.x); w[5] = bf_hi(b.x); w[6] = bf_lo(b.y); w[7] = bf_hi(b.y);
       } else {
         *reinterpret_cast<float4 *>(&w[0]) =
             *reinterpret_cast<const float4 *>((const float *)p.norm_w + c);
