@@ -117,6 +117,40 @@ def test_q4_rows(oracle, rows, cols, values):
     assert (off <= bound + 1e-45).all(), (off / np.maximum(bound, 1e-300)).max()
 
 
+@pytest.mark.parametrize("rows,cols", [(8, 256), (2372, 512), (300, 11008), (64, 4096)])
+@pytest.mark.parametrize("far", [1e8, 1e13, 1e30])
+def test_q4_values_far_apart(oracle, rows, cols, far):
+    """One of 32 values far above the others, and most rows without a weight for it: what is
+    left is as exact as x is in f32. A lane adds one of 32 products, the lanes five times, and
+    the norm's factor and y are one rounding each."""
+    w, s = oracle.quant_inputs("q4", rows, cols, 5)
+    codes = (w.view(np.uint32).reshape(rows, -1, 1) >> np.arange(0, 32, 4, dtype=np.uint32)) & 15
+    codes = codes.reshape(rows, cols).copy()
+    codes[rows // 8:, 3::32] = 8
+    w = (codes.reshape(rows, -1, 8) << np.arange(0, 32, 4, dtype=np.uint32)).sum(
+        2, dtype=np.uint32).reshape(w.shape)
+    x = oracle.random_f32(cols, 6, 1.0)
+    x[3::32] *= np.float32(far)
+    scales = np.repeat(s.view(np.float16).reshape(rows, -1).astype(np.float64), 32, axis=1)
+    weights = (codes.astype(np.float64) - 8.0) * scales
+    want, size = weights @ x.astype(np.float64), np.abs(weights) @ np.abs(x.astype(np.float64))
+    bound = (cols // 32 + 7) * 2.0 ** -24 * size
+    tw, ts, tx = dev(w.astype(np.uint32).view(np.int32)), dev(s), dev(x)
+    ty = abi.DeviceTensor.empty((rows,), abi.F32)
+    ops.nn_matvec_quant("q4", ty, tw, ts, tx, rows, cols)
+    assert (np.abs(ty.to_host().astype(np.float64) - want) <= bound).all()
+    y0 = oracle.random_f32(rows, 4, 1.0)
+    ta = dev(y0)
+    ops.nn_matvec_quant("q4", ta, tw, ts, tx, rows, cols, add=True)
+    assert (np.abs(ta.to_host().astype(np.float64) - want - y0) <= bound + 2.0 ** -24 *
+            np.abs(y0)).all()
+    half = rows // 2
+    to = abi.DeviceTensor.empty((half,), abi.F32)
+    ops.nn_swiglu_quant("q4", to, tw, ts, tx, half, cols)
+    g, u = want[rows // 8:half], want[rows // 8 + half:]
+    close(to.to_host()[rows // 8:], g / (1 + np.exp(-g)) * u)
+
+
 def test_q4_not_a_number(oracle):
     """An infinity or a NaN in x makes every row NaN."""
     rows, cols = 8, 512

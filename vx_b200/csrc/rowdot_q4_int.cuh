@@ -11,7 +11,11 @@
  * below 2^-38 of the largest of its 32.  Off from 64 bits, x from N(0, 1): 4096 x 4096
  * 4.9e-8, 4096 x 11008 6.2e-8 (three bf16 terms of x on bf16 mma.sync, which this
  * replaced: 1.0e-7, 1.4e-7); with one x of 10^6 whose weights are all 0: 1.0e-7, 8.7e-8
- * (1.0e-7, 1.4e-7; four bytes alone: 2.8e-5).
+ * (1.0e-7, 1.4e-7; four bytes alone: 2.8e-5).  With values further apart the small ones
+ * would lose what a row without a weight for the large one shows (all of it where that is
+ * 10^12): where four neighbours lie 2^-17 below the largest of their 32, or further, every
+ * sum of the launch is made from x in f32 instead (4096 x 4096 in 55 us, not 4.8).  Looking
+ * for them takes 0.8 % of a step (sixteen tokens of the 7B-shaped decoder 24.2 -> 24.4 ms).
  *
  * Bytes because of what it takes to unpack a code: eight codes are 4-bit fields of a word;
  * the odd ones in place and the even ones shifted up by four are bytes 16 * code, and
@@ -91,12 +95,37 @@ inline size_t q4_int_smem(int stages, int cols, const Q4IntPlan &plan) {
          sizeof(float2) * plan.round * plan.slices * 8;
 }
 
+/* The two results of an item with x in f32 as it is; every lane has them. A column of both
+   rows to a lane at a time, and rolled: a case that hardly occurs, whose instructions cost
+   every launch as they come from HBM with the others (eight columns at a time four times as
+   fast here, and 1.5 % of a step). */
+template <int EPI>
+__device__ __forceinline__ float2 item_of_wide_x(const RowDotParams &p, int item) {
+  const ItemRows it = item_rows<Q4W, EPI>(p, item);
+  const int lane = threadIdx.x & 31;
+  float t[2] = {0.0f, 0.0f};
+#pragma unroll 1
+  for (int c = lane; c < p.cols; c += 32) {
+    float x = p.x[c];
+    if (p.norm_w)
+      x *= p.norm_bf16 ? bf16_at(p.norm_w, c) : ((const float *)p.norm_w)[c];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const char *codes = h && it.r1 ? it.r1 : it.r0, *scales = h && it.r1 ? it.sc1 : it.sc0;
+      const int code = ((const unsigned char *)codes)[c / 2] >> (c % 2 * 4) & 15;
+      t[h] = fmaf((float)(code - 8) * __half2float(((const __half *)scales)[c / 32]), x, t[h]);
+    }
+  }
+  return make_float2(warp_sum(t[0]), warp_sum(t[1]));
+}
+
 template <int EPI, int STAGES>
 __global__ void __launch_bounds__(I_WARPS * 32, 2)
 q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char *smem = smem_raw + ((128 - (ptx::smem_addr(smem_raw) & 127)) & 127);
   __shared__ float ssq[I_WARPS];
+  __shared__ __align__(16) int wide[I_WARPS]; /* x too far apart for whole numbers */
   const int cols = p.cols;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -230,6 +259,7 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
   /* ---- x, times the norm's gains if any, as whole numbers: a thread takes eight
      columns, four threads the 32 that share a factor ---- */
   float ss = 0.0f;
+  bool far = false;
   constexpr int kApart = I_WARPS * 32 * 8;
   for (int c0 = threadIdx.x * 8; c0 < cols; c0 += 2 * kApart) {
     /* two runs' loads in flight at once: a trip to L2 is half a microsecond */
@@ -269,16 +299,22 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
           ss = fmaf(v[j], v[j], ss);
           v[j] *= ws[k][j];
         }
-      float top = max_nan(fabsf(v[0]), fabsf(v[1]));
+      float four[2];
 #pragma unroll
-      for (int j = 2; j < 8; ++j)
-        top = max_nan(top, fabsf(v[j]));
+      for (int h = 0; h < 2; ++h)
+        four[h] = max_nan(max_nan(fabsf(v[4 * h]), fabsf(v[4 * h + 1])),
+                          max_nan(fabsf(v[4 * h + 2]), fabsf(v[4 * h + 3])));
+      float top = max_nan(four[0], four[1]);
       top = max_nan(top, __shfl_xor_sync(0xffffffffu, top, 1));
       top = max_nan(top, __shfl_xor_sync(0xffffffffu, top, 2));
       /* 2^s brings the largest into [2^29, 2^30). Below 2^-117 s stays: what is cut then
          lies below the smallest f32. In two factors: 2^s itself may be above the largest
          f32. Infinities and NaN make the factor, and so every result, NaN. */
       const int e = max((int)(__float_as_uint(top) >> 23 & 255u), 10);
+      /* four neighbours, not all 0, that lie 2^-17 below the largest or further: the sums
+         are then made from x itself */
+      const uint32_t low = e == 255 ? 0u : (uint32_t)max(e - 16, 0) << 23;
+      far |= __float_as_uint(four[0]) - 1u < low || __float_as_uint(four[1]) - 1u < low;
       if (e < 64)
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -316,6 +352,9 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
                                    : __uint_as_float((uint32_t)(e - 9) << 23);
     }
   }
+  far = __any_sync(0xffffffffu, far);
+  if (lane == 0)
+    wide[warp] = far;
   if (p.norm_w) {
     ss = warp_sum(ss);
     if (lane == 0)
@@ -404,6 +443,18 @@ q4_int_kernel(const RowDotParams p, const Q4IntPlan plan) {
         parts[((tile - round) * plan.slices + slice) * 8 + g] = make_float2(v, w);
     }
     __syncthreads();
+    const int4 far0 = *reinterpret_cast<const int4 *>(&wide[0]);
+    const int4 far1 = *reinterpret_cast<const int4 *>(&wide[4]);
+    if (far0.x | far0.y | far0.z | far0.w | far1.x | far1.y | far1.z | far1.w) {
+#pragma unroll 1
+      for (int i = round * 8 + warp; i < end * 8 && first + i < last; i += I_WARPS) {
+        const float2 t = item_of_wide_x<EPI>(p, first + i);
+        if (lane < plan.slices) /* whose sum over the slices it is then */
+          parts[((i / 8 - round) * plan.slices + lane) * 8 + i % 8] =
+              lane ? make_float2(0.0f, 0.0f) : t;
+      }
+      __syncthreads();
+    }
     const int item = first + round * 8 + threadIdx.x;
     if ((int)threadIdx.x < plan.round * 8 && item < last) {
       const float2 *at = parts + (threadIdx.x >> 3) * plan.slices * 8 + (threadIdx.x & 7);
