@@ -650,20 +650,33 @@ const char *attention_decode(const AttnArgs &a, cudaStream_t stream) {
               (heads * cl >= 3 * sm_count() &&
                heads <= resident_clusters((const void *)kernel, cl, 4 * 32)));
     };
-    /* One block of 16 warps a head where it is soon done with the longest cache this launch
-       may see, 100 KB of it: the small f32 decoder (six heads of 48, 256 positions) saves
-       two meetings of a cluster a layer, 8.2 -> 7.5 ms for 64 tokens. */
-    const bool one_block = (int64_t)(a.max_pos + 1) * a.head_dim * 8 <= 100 * 1024;
-    /* Four of 16 warps where those are one wave and eight of eight would be two: an SM holds
-       two of these, but clusters of eight do not divide the SMs of a GPC, and of 32 heads at
-       1000 positions the last ones began 8 us after the first (82.2 us a layer of the
-       7B-shaped bf16 step, so 77.5; at 520 to 650 387.0 and 389.2 tokens/s). */
-    const bool one_wave = 4 * heads <= sm_count() && 8 * heads > sm_count();
+    /* One block of 16 warps a head, without the two meetings of a cluster, where it is soon
+       done with all positions this launch may see: 256 where they are fetched ahead of the
+       kernel in front (and at most 100 KB of a head), else 48. Decoders of 6 to 64 heads of
+       16 to 48 values, us a layer, one block / eight: at 10 positions 18.0 / 19.1 to 21.7 /
+       24.2, at 220 19.4 / 19.3 to 23.1 / 24.5; beyond 256 it loses (heads of 24 at 400 21.8 /
+       19.3, of 16 at 700 24.3 / 19.2). By itself, heads of 64 and 128, 8 to 64 of them: at 16
+       positions 2.9 / 3.8, at 48 3.4 / 3.9 to 4.3 / 4.5, at 64 3.6 / 3.9 to 5.1 / 5.1 and, 32
+       of 128, 4.9 / 4.6, at 200 5.3 / 4.3 to 10.2 / 8.1. (The 100 KB keep decoders with heads
+       of 64 and 128 on the clusters: 8 and 32 heads of one sequence would take 1.2 to 1.5 us
+       less at 10 positions and 0 to 0.2 at 220; sequences by the dozen are not measured.) */
+    const bool one_block = a.max_pos < (a.rows_settled ? 256 : 48) &&
+                           (int64_t)(a.max_pos + 1) * a.head_dim * 8 <= 100 * 1024;
+    /* Four of 16 warps where those are one wave and eight of eight are not: an SM holds two
+       of the latter, but clusters of eight do not divide the SMs of a GPC. A layer of a bf16
+       decoder, us, four / eight: 31 heads at 10, 1000 and 3000 positions 27.1 / 28.9, 31.8 /
+       33.9, 41.2 / 45.4; 33 27.4 / 29.9, 32.1 / 35.2, 42.0 / 48.8. 30 heads of eight are one
+       wave too (the runtime says 33): 26.6 / 26.7, 31.3 / 31.2, 40.5 / 40.2, and 20 at 3000
+       35.1 / 34.3; 34 of four are not: 30.9 / 30.7, 37.1 / 36.5, 53.0 / 51.2. */
+    auto one_wave = [&](auto kernel) {
+      return 64 * heads > 13 * sm_count() &&
+             heads <= resident_clusters((const void *)kernel, 4, 16 * 32);
+    };
     auto of_heads = [&](auto gh_c) {
       constexpr int GH = decltype(gh_c)::value;
       if (one_block && !is_pinned)
         go(attention_cluster_kernel<GH, 16, 1>, 1, 16);
-      else if (one_wave && !is_pinned)
+      else if (!is_pinned && one_wave(attention_cluster_kernel<GH, 16, 4>))
         go(attention_cluster_kernel<GH, 16, 4>, 4, 16);
       else if (few(attention_cluster_kernel<GH, 4, 1>, 1))
         go(attention_cluster_kernel<GH, 4, 1>, 1, 4);
