@@ -18,8 +18,8 @@
  *
  * What bounds it: of few tiles the trips to memory and the launch, of many the FP32 pipe,
  * 1.7 us for 128 of K of each tile of an SM.  In a graph, us, the terms' kernel in
- * brackets: 64^3 4.1 (6.9), 257 x 300 x 190 9.1 (11.6), 64 x 64 x 3072 9.6 (18.0), 512 x 512
- * x 128 6.8 (9.4), 512^3 16.5 (19.6); 1024^3 would take 92 (22.4).
+ * brackets: 64^3 4.1 (5.8), 257 x 300 x 190 8.8 (10.5), 64 x 64 x 2048 7.7 (12.9), 512 x 512
+ * x 128 6.9 (8.3), 512^3 17.1 (18.3); 1024 x 1024 x 512 would take 54 (13.9).
  */
 #include "kernels.h"
 #include "launch.cuh"
@@ -263,18 +263,23 @@ int runs_of(int64_t m, int64_t n, int64_t k) {
 
 } // namespace
 
-/* Microseconds, about: 1.7 for 128 of K of each tile that an SM has, 3.2 for a launch, 1.5
-   for the meeting of a cluster. Measured 4.1 / 9.1 / 5.9 / 9.6 / 7.5 / 6.8 / 16.5 / 29 at
-   64^3, 257 x 300 x 190, 64 x 64 x 1024, 64 x 64 x 3072, 256^3, 512 x 512 x 128, 512^3 and
-   1024 x 1024 x 256, where this gives 4.9 / 6.6 / 6.4 / 9.8 / 6.4 / 6.6 / 16.8 / 27.0. */
+/* Microseconds, about, one call after another: 1.73 for 128 of K of each tile that an SM has,
+   3.2 for a launch, 1.5 for the meeting of a cluster, 0.9 for each tile an SM has after its
+   first two. From half as many blocks as SMs on, some SM has two: blocks begin beside those of
+   the call before, on what SMs that leaves. Measured 4.1 / 5.9 / 8.7 / 8.8 / 6.9 / 17.1 / 14.2 /
+   32.0 at 64^3, 64 x 64 x 1024, 320 x 320 x 256, 257 x 300 x 190, 512 x 512 x 128, 512^3,
+   576 x 576 x 256 and 768 x 768 x 512, where this gives 4.9 / 6.4 / 10.1 / 10.1 / 6.7 / 17.0 /
+   14.5 / 32.7. */
 double gemm_f32_small_us(int64_t m, int64_t n, int64_t k) {
   if (m > 65535ll * TILE || n > INT32_MAX - TILE || k > INT32_MAX - 4 * KC)
     return HUGE_VAL;
   const int64_t z = runs_of(m, n, k);
   const int64_t blocks = ((m + TILE - 1) / TILE) * ((n + TILE - 1) / TILE) * z;
   const int64_t chunks = ((k + z - 1) / z + KC - 1) / KC;
-  return 3.2 + (z > 1 ? 1.5 : 0.0) +
-         1.7 * (double)((blocks + sm_count() - 1) / sm_count() * chunks);
+  const int64_t rounds = (blocks + sm_count() - 1) / sm_count();
+  const int64_t on_an_sm = 2 * blocks <= sm_count() ? 1 : rounds < 2 ? 2 : rounds;
+  return 3.2 + (z > 1 ? 1.5 : 0.0) + 1.73 * (double)(on_an_sm * chunks) +
+         (on_an_sm > 2 ? 0.9 * (double)(on_an_sm - 2) : 0.0);
 }
 
 const char *gemm_f32_small(const float *a, int64_t lda, const float *b, int64_t ldb, float *c,
