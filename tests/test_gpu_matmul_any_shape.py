@@ -124,6 +124,58 @@ def test_f32_values_that_three_bf16_terms_cannot_carry(k):
     assert np.abs(got[fine] - want[fine]).max() <= k * 2.0 ** -23
 
 
+# What the time model sends to small tiles, on the terms' kernel: VXB_F32_TENSOR=1 keeps f32
+# on the tensor cores.
+@pytest.fixture
+def on_tensor_cores(monkeypatch):
+    monkeypatch.setenv("VXB_F32_TENSOR", "1")
+
+
+@pytest.mark.parametrize("m,n,k,off,pad", F32)
+def test_f32_products_of_any_shape_on_tensor_cores(on_tensor_cores, m, n, k, off, pad):
+    test_f32_products_of_any_shape(m, n, k, off, pad)
+
+
+@pytest.mark.parametrize("k", [150, 1100])
+def test_f32_values_that_terms_cannot_carry_on_tensor_cores(on_tensor_cores, k):
+    test_f32_values_that_three_bf16_terms_cannot_carry(k)
+
+
+def test_f32_values_of_every_size_on_tensor_cores(on_tensor_cores):
+    test_f32_values_of_every_size_that_terms_carry()
+
+
+# sizes that go there by themselves: a tile's own K, clusters of two and four, rows off the
+# 16- and 8-byte grids
+@pytest.mark.parametrize("m,n,k,off,pad", [(600, 600, 641, 1, 1), (1030, 520, 577, 2, 2),
+                                           (1300, 1100, 100, 3, 3), (330, 300, 2500, 0, 2)])
+def test_f32_large_tiles_of_special_values(m, n, k, off, pad):
+    """Infinities, NaN, a product that overflows, a row of subnormals and whole numbers, in
+    views off the grid."""
+    rng = np.random.default_rng(m + k)
+    a = rng.integers(-8, 9, (m, k)).astype(np.float32)
+    b = rng.integers(-8, 9, (k, n)).astype(np.float32)
+    args = dict(offsets=(off, off, off), pads=(pad, pad, pad))
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    assert np.array_equal(product(a, b, m, n, k, abi.F32, **args), want)
+    a[3, 5], a[m - 1, 0] = np.inf, 1e30
+    b[9, 17], b[0, n - 1] = np.nan, 1e30
+    a[20] = rng.uniform(-1, 1, k) * 1e-39
+    got = product(a, b, m, n, k, abi.F32, **args)
+    with np.errstate(all="ignore"):
+        want = a.astype(np.float64) @ b.astype(np.float64)
+        want32 = want.astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(want32))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want32))
+    assert np.array_equal(np.isneginf(got), np.isneginf(want32))
+    fine = np.isfinite(want32) & (np.abs(want) < 1e20)
+    size = np.abs(np.where(np.isfinite(a), a, 0)).astype(np.float64) @ \
+        np.abs(np.where(np.isfinite(b), b, 0)).astype(np.float64)
+    # a result is rounded once more where it is subnormal
+    bound = (1e-6 * size + 2.0 ** -149)[fine]
+    assert (np.abs(got[fine] - want[fine]) <= bound).all()
+
+
 # runs of K (few tiles), copies (odd rows, views off the grid) of A, of B and of both, a C
 # whose rows begin anywhere, the plain kernel's sizes, tiles of 128 and of 256 columns
 B16 = [(100, 100, 4000, 0, 0), (128, 256, 1000, 0, 0), (129, 257, 777, 0, 0),

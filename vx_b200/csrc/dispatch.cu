@@ -656,21 +656,22 @@ void gemm_on_device(const vx_gemm_plan &p, const Staged &a, const Staged &b,
   switch (p.dtype) {
   case VX_DTYPE_F32: {
     /* on the FP32 pipe in small tiles, or on the tensor cores as exact bf16 terms
-       (VXB_F32_TENSOR=0: always the FP32 pipe, in large tiles): the terms made inside the
-       kernel, or beforehand for whole tiles of large products, whichever takes less time.
+       (VXB_F32_TENSOR=0: always the FP32 pipe, in large tiles; 1: always the tensor cores):
+       the terms made inside the kernel, or beforehand for whole tiles of large products,
+       whichever takes less time.
        The first has to be 4 us ahead of the second, whose time model is that of a call by
        itself: one call after another takes 4 to 5 us less (512 x 512 x 256 8.7, the model
        12.7), and the small tiles' model is that of those. Of 80 sizes on both sides of the
        line, 64^3 to 1024^2 x 512, three go to the slower one, which takes 8 to 10 % longer. */
-    const char *off = getenv("VXB_F32_TENSOR");
-    if (off && off[0] == '0') {
+    const char *pin = getenv("VXB_F32_TENSOR");
+    if (pin && pin[0] == '0') {
       why = vxb::gemm_f32((const float *)a.ptr, a.row_stride,
                           (const float *)b.ptr, b.row_stride, (float *)c, ldc,
                           p.m, p.n, p.k, t_stream);
       break;
     }
     const double tile_us = vxb::gemm_f32_tile_us(p.m, p.n, p.k);
-    if (vxb::gemm_f32_small_us(p.m, p.n, p.k) + 4.0 < tile_us) {
+    if (!(pin && pin[0] == '1') && vxb::gemm_f32_small_us(p.m, p.n, p.k) + 4.0 < tile_us) {
       why = vxb::gemm_f32_small((const float *)a.ptr, a.row_stride, (const float *)b.ptr,
                                 b.row_stride, (float *)c, ldc, p.m, p.n, p.k, t_stream);
       break;
