@@ -224,6 +224,23 @@ def test_f32_products_of_one_sign(m, n, k):
     assert rel(product(a, b, m, n, k, abi.F32), want) <= 1.4 * 8 * 2.2e-8
 
 
+def test_f32_products_from_several_threads_at_once():
+    """Clusters of two, four and eight blocks, whose number on the GPU the first call asks for."""
+    import concurrent.futures
+    rng = np.random.default_rng(8)
+    jobs = []
+    for m, n, k in [(1030, 520, 577), (600, 600, 641), (330, 300, 2500), (257, 300, 190)]:
+        a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+        b = rng.uniform(-1, 1, (k, n)).astype(np.float32)
+        jobs.append((a, b, m, n, k, a.astype(np.float64) @ b.astype(np.float64)))
+
+    def one(i):
+        a, b, m, n, k, want = jobs[i % len(jobs)]
+        return rel(product(a, b, m, n, k, abi.F32), want)
+    with concurrent.futures.ThreadPoolExecutor(8) as pool:
+        assert max(pool.map(one, range(32))) <= 1e-6
+
+
 def microseconds(a, b, m, n, k):
     """Of one product of device tensors, the least of five runs of twenty."""
     import torch

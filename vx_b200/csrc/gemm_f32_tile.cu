@@ -375,30 +375,13 @@ constexpr int64_t kMostRowTiles = 65535; /* in a grid's second dimension */
 
 /* How many clusters of z blocks the GPU holds at once: they do not divide the SMs of a
    GPC. */
-int64_t resident_clusters(int z) {
-  static int known[4] = {0, 0, 0, 0}; /* of 2, 4, 8 blocks; every thread finds the same */
-  const int at = z == 2 ? 1 : z == 4 ? 2 : 3;
-  if (!known[at]) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)z);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)z;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (allow_dynamic_smem((const void *)gemm_f32_tile_kernel, SMEM_BYTES) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, gemm_f32_tile_kernel, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      n = sm_count() / z > 1 ? sm_count() / z : 1;
-    }
-    known[at] = n;
+int64_t clusters_at_once(int z) {
+  if (allow_dynamic_smem((const void *)gemm_f32_tile_kernel, SMEM_BYTES) == cudaSuccess) {
+    const int n = resident_clusters((const void *)gemm_f32_tile_kernel, z, THREADS, SMEM_BYTES);
+    if (n > 0)
+      return n;
   }
-  return known[at];
+  return sm_count() / z > 1 ? sm_count() / z : 1;
 }
 
 /* How many blocks share a tile: more while the chip has room for them, each keeps a block
@@ -410,7 +393,7 @@ int blocks_of_tile(int64_t m, int64_t n, int64_t k) {
   const int64_t k_blocks = (k + BK - 1) / BK;
   int z = 1;
   while (z < 8 && tiles * z * 2 <= sm_count() && k_blocks >= 2 * z &&
-         (k_blocks < 3 * z || tiles <= resident_clusters(2 * z)))
+         (k_blocks < 3 * z || tiles <= clusters_at_once(2 * z)))
     z *= 2;
   return z;
 }
@@ -428,7 +411,7 @@ double gemm_f32_tile_us(int64_t m, int64_t n, int64_t k) {
     return HUGE_VAL;
   const int64_t z = blocks_of_tile(m, n, k);
   const int64_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-  const int64_t at_once = z > 1 ? resident_clusters((int)z) : sm_count();
+  const int64_t at_once = z > 1 ? clusters_at_once((int)z) : sm_count();
   const int64_t k_blocks = ((k + BK - 1) / BK + z - 1) / z;
   return 3.6 + (double)((tiles + at_once - 1) / at_once) * (7.4 + 1.7 * k_blocks);
 }

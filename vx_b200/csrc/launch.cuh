@@ -24,6 +24,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 namespace vxb {
@@ -76,6 +77,39 @@ inline void prefer_shared_memory(const void *kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
   done = true;
+}
+
+/* How many clusters of `cluster` blocks the current GPU holds at once; 0: not known (and
+   asked again by the next call). Any thread may ask. */
+inline int resident_clusters(const void *kernel, int cluster, int threads, size_t smem = 0) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void *, int, int>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess)
+    return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(kernel, cluster, dev);
+  const auto hit = known.find(key);
+  if (hit != known.end())
+    return hit->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cluster);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  known[key] = n;
+  return n;
 }
 
 inline bool chain_enabled() {

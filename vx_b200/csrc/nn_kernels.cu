@@ -563,36 +563,6 @@ size_t attn_scratch_floats(int batch, int q_heads, int head_dim, int max_seq,
          (head_dim + 2);
 }
 
-/* How many clusters of `cl` blocks the current GPU holds at once. */
-static int resident_clusters(const void *kernel, int cl, int threads) {
-  static std::mutex mu;
-  static std::map<std::pair<const void *, int>, int> asked;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_pair(kernel, dev);
-  const auto hit = asked.find(key);
-  if (hit != asked.end())
-    return hit->second;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(threads);
-  cfg.gridDim = dim3(cl);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cl;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    n = 0;
-  }
-  asked[key] = n;
-  return n;
-}
-
 const char *attention_decode(const AttnArgs &a, cudaStream_t stream) {
   if (a.head_dim % 4 != 0 || a.head_dim > 128)
     return "head_dim must be a multiple of 4, and at most 128";
