@@ -52,7 +52,6 @@ size_t gemm_16_scratch_bytes(const void *, int64_t, const void *, int64_t, int64
 double gemm_f32_small_us(int64_t, int64_t, int64_t) { return 0.0; }
 double gemm_f32_tile_us(int64_t, int64_t, int64_t) { return 0.0; }
 double gemm_f32_split_us(int64_t, int64_t, int64_t, int64_t) { return 0.0; }
-bool batched_proj_leaves_norm(int) { return false; }
 size_t batched_proj_scratch_floats(int, int) { return 0; }
 size_t step_scratch_floats(int) { return 0; }
 int gemm_status(Stream) { return 0; }

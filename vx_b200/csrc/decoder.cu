@@ -466,13 +466,11 @@ void record_step(vx_decoder *d, int max_pos) {
     need(vxb::batched_proj(bp, s), what);
     launches += terms_ready ? 2 : 3;
   };
-  /* a residual projection leaves the next one's input, normalised */
-  const bool norm_left = d->mma && vxb::batched_proj_leaves_norm(c.dim);
   for (int l = 0; l < c.n_layers; ++l) {
     if (d->mma) {
       batched(4, d->wq[l], d->wk[l], d->wv[l], (d->q_local + 2 * d->kv_local) * hd,
               c.dim, d->x, d->attn_norm[l], d->q, (int64_t)d->q_local * hd,
-              d->bqkv[l], l, "q/k/v", norm_left && l > 0);
+              d->bqkv[l], l, "q/k/v", l > 0);
       vxb::AttnArgs ab{};
       ab.q = d->q;
       ab.k_cache = d->k_cache + l * d->cache_layer_stride;
@@ -492,16 +490,15 @@ void record_step(vx_decoder *d, int max_pos) {
       need(vxb::attention_decode(ab, s), "attention");
       ++launches;
       batched(1, d->wo[l], nullptr, nullptr, c.dim, d->q_local * hd, d->att,
-              nullptr, d->x, c.dim, nullptr, l, "the output projection", false,
-              norm_left, norm_left ? d->ffn_norm[l] : nullptr);
-      /* SwiGLU's finishing kernel leaves the down projection's input as terms */
+              nullptr, d->x, c.dim, nullptr, l, "the output projection", false, true,
+              d->ffn_norm[l]);
+      /* a residual projection leaves the next one's input, normalised; SwiGLU's finishing
+         kernel the down projection's, as terms */
       batched(3, d->w_gate[l], d->w_up[l], nullptr, d->hidden_local, c.dim, d->x,
-              d->ffn_norm[l], d->h, d->hidden_local, nullptr, l, "gate/up", norm_left,
-              true);
+              d->ffn_norm[l], d->h, d->hidden_local, nullptr, l, "gate/up", true, true);
       const void *next = l + 1 < c.n_layers ? d->attn_norm[l + 1] : d->final_norm;
       batched(1, d->w_down[l], nullptr, nullptr, c.dim, d->hidden_local, d->h,
-              nullptr, d->x, c.dim, nullptr, l, "the down projection", true, norm_left,
-              norm_left ? next : nullptr);
+              nullptr, d->x, c.dim, nullptr, l, "the down projection", true, true, next);
       continue;
     }
     vxb::QkvArgs qa{};
@@ -615,7 +612,7 @@ void record_step(vx_decoder *d, int max_pos) {
   if (d->mma) {
     batched(0, d->lm_head, nullptr, nullptr, d->vocab_local, c.dim, d->x,
             d->final_norm, d->logits, d->vocab_local, nullptr, 0, "the logits",
-            norm_left && c.n_layers > 0);
+            c.n_layers > 0);
   } else {
   vxb::MatvecArgs la{};
   la.w = d->lm_head;

@@ -397,11 +397,10 @@ struct BatchedProj {
   /* chaining: x's terms are in xs already (left by the projection before);
      leave this projection's output there as terms for the next one: mode 3, SwiGLU's
      output is the down projection's input; mode 1, the next one reads y normalised with
-     the gains next_norm_w (batched_proj_leaves_norm says for which rows). */
+     the gains next_norm_w. */
   int x_terms_ready, next_terms;
   const void *next_norm_w;
 };
-bool batched_proj_leaves_norm(int rows);
 const char *batched_proj_refusal(const BatchedProj &a);
 size_t batched_proj_scratch_floats(int rows_max, int batch);
 const char *batched_proj(const BatchedProj &a, cudaStream_t stream);

@@ -221,8 +221,9 @@ const char *rows_fan_finish(const float *partials, int splits, int t, int n,
                             int out_col, cudaStream_t stream) {
   if ((n | out.k_row | out.gate_row | out.up_row | out_cols | out_col) % 8 != 0)
     return "the parts of an input projection are multiples of 8 rows";
-  launch_chained(fan_finish_kernel, dim3(t, (n / 8 + 255) / 256), dim3(256), 0, stream, partials, splits, t, n, out, positions, q_out, q_stride,
-                 k_cache, (__nv_bfloat16 *)terms, out_cols, out_col);
+  launch_chained(fan_finish_kernel, dim3(t, (n / 8 + 255) / 256), dim3(256), 0, stream, partials,
+                 splits, t, n, out, positions, q_out, q_stride, k_cache, (__nv_bfloat16 *)terms,
+                 out_cols, out_col);
   return check_launch("the parts of an input projection");
 }
 

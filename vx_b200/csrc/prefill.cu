@@ -303,49 +303,10 @@ norm_terms_kernel(__nv_bfloat16 *terms, const float *x, const NormGain w, int di
 
 /* After the output or the down projection, when an RMSNorm follows: x[t] += the
    product, and the terms of the normalised x[t] for the next GEMM, in one pass
-   over the row (the sums in the order of residual_finish_kernel and
-   norm_terms_kernel). One block per position; dim <= 256 * 32. */
-__global__ void __launch_bounds__(256)
-residual_norm_kernel(__nv_bfloat16 *terms, float *x, const float *partials,
-                     int splits, int t_count, const NormGain w, int dim, float eps) {
-  __shared__ float red[8];
-  chain_release();
-  chain_wait();
-  const int64_t t = blockIdx.x;
-  float *xr = x + t * dim;
-  constexpr int PER = 32;
-  float v[PER];
-  float ss = 0.0f;
-#pragma unroll
-  for (int k = 0; k < PER; ++k) {
-    const int i = threadIdx.x + k * 256;
-    v[k] = 0.0f;
-    if (i < dim) {
-      v[k] = xr[i] + sum_runs(partials, splits, t_count, dim, t, i);
-      xr[i] = v[k];
-      ss = fmaf(v[k], v[k], ss);
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1)
-    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if ((threadIdx.x & 31) == 0)
-    red[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  float total = 0.0f;
-  for (int k = 0; k < 8; ++k) /* fixed order */
-    total += red[k];
-  const float inv = 1.0f / sqrtf(total / (float)(w.n ? w.n : dim) + eps);
-#pragma unroll
-  for (int k = 0; k < PER; ++k) {
-    const int i = threadIdx.x + k * 256;
-    if (i < dim)
-      store_terms(terms, dim, t, i, v[k] * gain_at(w, i) * inv);
-  }
-}
-
-/* The same for rows of whole quads, at most QUADS of them a thread, whose loads of a run are
-   in flight together. Value by value, a trip to L2 after another, 499 rows of 4096 took 28
-   us; so 10. */
+   over the row (the runs in the order of residual_finish_kernel). One block per
+   position; dim is a multiple of 4, at most QUADS quads a thread, whose loads of a run
+   are in flight together. Value by value, a trip to L2 after another, 499 rows of 4096
+   took 28 us; so 10. */
 template <int QUADS>
 __global__ void __launch_bounds__(256)
 residual_norm_quads_kernel(__nv_bfloat16 *terms, float *x, const float *partials, int splits,
@@ -775,8 +736,9 @@ const char *rows_qkv_finish(const float *partials, int splits, int t, int q_head
   if (hd % 8 != 0)
     return "the multi-position RoPE takes head_dim in multiples of 8";
   const int n = (q_heads + 2 * kv_heads) * (hd / 8);
-  launch_chained(qkv_finish_kernel, dim3(t, (n + 255) / 256), dim3(256), 0, stream, partials, splits, t, q_heads, kv_heads, hd, bias, cos_t,
-                 sin_t, first_pos, q_out, k_cache, v_cache);
+  launch_chained(qkv_finish_kernel, dim3(t, (n + 255) / 256), dim3(256), 0, stream, partials,
+                 splits, t, q_heads, kv_heads, hd, bias, cos_t, sin_t, first_pos, q_out, k_cache,
+                 v_cache);
   return last_launch("the multi-position RoPE and cache store");
 }
 
@@ -793,13 +755,12 @@ const char *rows_residual_norm(void *terms, float *x, const float *partials,
                                cudaStream_t stream) {
   if (dim > 256 * 32)
     return "the fused residual and RMSNorm take rows of at most 8192 values";
-  const bool whole = dim % 4 == 0 && !(((uintptr_t)x | (uintptr_t)partials) & 15) &&
-                     !((uintptr_t)terms & 7);
-  auto kernel = !whole             ? residual_norm_kernel
-                : dim <= 4 * 4 * 256 ? residual_norm_quads_kernel<4>
-                                     : residual_norm_quads_kernel<8>;
-  launch_chained(kernel, dim3(t), dim3(256), 0, stream, (__nv_bfloat16 *)terms, x, partials,
-                 splits, t, w, dim, eps);
+  if (dim % 4 != 0 || (((uintptr_t)x | (uintptr_t)partials) & 15) || ((uintptr_t)terms & 7))
+    return "the fused residual and RMSNorm take rows of whole quads";
+  launch_chained(dim <= 4 * 4 * 256 ? residual_norm_quads_kernel<4>
+                                    : residual_norm_quads_kernel<8>,
+                 dim3(t), dim3(256), 0, stream, (__nv_bfloat16 *)terms, x, partials, splits, t,
+                 w, dim, eps);
   return last_launch("the multi-position residual add and RMSNorm");
 }
 

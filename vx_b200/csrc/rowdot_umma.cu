@@ -632,10 +632,6 @@ const char *batched_proj_refusal(const BatchedProj &a) {
   return nullptr;
 }
 
-bool batched_proj_leaves_norm(int rows) {
-  return rows % 2 == 0;
-}
-
 size_t batched_proj_scratch_floats(int rows_max, int batch) {
   /* up to 16 runs of [batch][rows rounded up to 128] */
   return (size_t)16 * batch * ((rows_max + 127) / 128 * 128);
@@ -675,7 +671,7 @@ const char *batched_proj(const BatchedProj &a, cudaStream_t stream) {
   if (a.next_terms && a.mode != 3 && (a.mode != 1 || !a.next_norm_w))
     return "only the SwiGLU and the residual projections can leave terms";
   if (a.next_terms && a.mode == 1 &&
-      (!batched_proj_leaves_norm(a.rows) || a.y_stride % 2 != 0 ||
+      (a.rows % 2 != 0 || a.y_stride % 2 != 0 ||
        (((uintptr_t)a.y | (uintptr_t)a.xs) & 7)))
     return "terms of a normalised row need pairs of values";
   int64_t rows0 = a.rows, rows1 = 0, rows2 = 0; /* rows of the three matrices */
