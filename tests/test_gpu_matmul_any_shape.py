@@ -71,16 +71,38 @@ SMALL = [(1, 1, 1, 0, 0), (31, 33, 3, 1, 0), (32, 32, 128, 0, 0), (33, 65, 129, 
 
 @pytest.mark.parametrize("m,n,k,off,pad", SMALL)
 def test_f32_products_in_small_tiles(m, n, k, off, pad):
-    """A sum of four products, two of those, the exact sum of these sums and one last
-    rounding: six roundings of at most 2^-24 of the sum of magnitudes, and what the
-    rest's own sum loses, 2^-24 of 2^-24 of it for each eight of K."""
+    """A sum of four products (four roundings), two of those (one), the sum of these sums with
+    its rest (one, where eight products are more than what is there already) and the last
+    one: seven roundings of at most 2^-24 of the sum of magnitudes, and what the rest's own
+    sum loses, 2^-24 of 2^-24 of it for each eight of K."""
     rng = np.random.default_rng(m * n + k)
     a = rng.uniform(-1, 1, (m, k)).astype(np.float32)
     b = (rng.uniform(-1, 1, (k, n)) * 10.0 ** rng.uniform(-3, 3, (k, 1))).astype(np.float32)
     got = product(a, b, m, n, k, abi.F32, offsets=(off, off, off), pads=(pad, pad, pad))
     want = a.astype(np.float64) @ b.astype(np.float64)
     size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
-    assert (np.abs(got - want) <= (6 + k / 8 * 2.0 ** -24) * 2.0 ** -24 * size).all()
+    assert (np.abs(got - want) <= (7 + k / 8 * 2.0 ** -24) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("m,n,k,off,pad", SMALL)
+@pytest.mark.parametrize("order", ["growing", "cancelling"])
+def test_f32_small_tiles_whose_sums_grow_or_cancel(order, m, n, k, off, pad):
+    """Each eight products larger than all before them, or the second half of K taking the
+    first half's sum away: the same seven roundings."""
+    rng = np.random.default_rng(m * n + k)
+    a = rng.uniform(0.5, 1, (m, k)).astype(np.float32)
+    b = rng.uniform(0.5, 1, (k, n)).astype(np.float32)
+    at = np.arange(k)[:, None]
+    if order == "growing":
+        b = (b * 1.5 ** np.minimum(at % 128 // 4, 60)).astype(np.float32)
+    else:
+        half = k // 2
+        a[:, half:2 * half] = a[:, :half]
+        b[half:2 * half] = -b[:half] * np.float32(1 + 1e-5)
+    got = product(a, b, m, n, k, abi.F32, offsets=(off, off, off), pads=(pad, pad, pad))
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    size = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    assert (np.abs(got - want) <= (7 + k / 8 * 2.0 ** -24) * 2.0 ** -24 * size).all()
 
 
 # the 128 x 128 tiles alone and in clusters of two, four and eight

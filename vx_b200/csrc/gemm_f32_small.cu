@@ -3,14 +3,16 @@
  * The tensor-core kernel of gemm_f32_tile.cu splits every value into three terms and has
  * tiles of 128 x 128: nine of them for 257 x 300 x 190, which took 13.4 us, most of it a
  * tile's start and end.  Here a tile is 32 x 32, so that the same product has 90 blocks, and
- * a block's eight warps share its K: each takes 16 of every 128, with a lane's 8 x 4 results
- * in registers (12 loads from shared memory for 128 multiply-adds), and the warps' sums meet
- * in shared memory at the end.  Where there are few tiles, K is divided over a cluster of up
- * to eight blocks as well, whose sums meet through distributed shared memory in run order.
+ * a block's eight warps share it: two take the halves of its rows, four such pairs a quarter
+ * of every 128 of K each, with a lane's 4 x 4 results in registers (eight loads from shared
+ * memory for 64 multiply-adds), and the pairs' sums meet in shared memory at the end.  Where
+ * there are few tiles, K is divided over a cluster of up to eight blocks as well, whose sums
+ * meet through distributed shared memory in run order.
  * A and B come by cp.async into three stages of 128 of K.
  *
- * Four products are added in f32, two such sums, and those sums exactly: what an addition
- * rounds off is kept beside the sum (with 16 products in a row it was 9.8e-8 from 64 bits
+ * Four products are added in f32, two such sums, and those sums with what an addition rounds
+ * off kept beside the sum: all of it where the sum so far is the larger, all but 2^-24 of the
+ * eight products where they are (with 16 products in a row it was 9.8e-8 from 64 bits
  * at 257 x 300 x 190, where the terms are 9.3e-8; so 5.7e-8, and 2e-8 to 3e-8 for values of
  * one sign, where the terms are 7e-8 to 1.5e-7).  Groups of warps and blocks add up in 64
  * bits.  B is multiplied by 2^24, which keeps products below the smallest f32; a tile in
@@ -79,8 +81,10 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
         "l"(*reinterpret_cast<const unsigned long long *>(&a)));
   return *reinterpret_cast<float2 *>(&d);
 }
-/* sum + x, and what its rounding takes off is added to `rest` (Dekker's sum of two, which
-   is exact where x is the smaller). */
+/* sum + x, and what its rounding takes off is added to `rest` (Dekker's sum of two: exact
+   where x is the smaller; else t - sum may round, by at most 2^-24 of x. The form that is
+   exact for any order takes three more operations, and the products in x have lost as much
+   by then). */
 __device__ __forceinline__ void add_with_rest(float2 &sum, float2 &rest, const float2 x) {
   const float2 t = add2(sum, x);
   rest = add2(rest, sub2(x, sub2(t, sum)));
