@@ -107,6 +107,7 @@ def test_f32_on_the_tensor_cores_is_as_good_as_the_fp32_kernel(m, n, k, monkeypa
     a = (rng.uniform(-1, 1, (m, k)) * np.exp(rng.uniform(-6, 6, (m, k)))).astype(np.float32)
     b = (rng.uniform(-1, 1, (k, n)) * np.exp(rng.uniform(-6, 6, (k, n)))).astype(np.float32)
     want = a.astype(np.float64) @ b.astype(np.float64)
+    monkeypatch.setenv("VXB_F32_TENSOR", "1")
     split = device_matmul(a, b)
     monkeypatch.setenv("VXB_F32_TENSOR", "0")
     plain = device_matmul(a, b)
@@ -117,9 +118,10 @@ def test_f32_on_the_tensor_cores_is_as_good_as_the_fp32_kernel(m, n, k, monkeypa
     assert not np.array_equal(split, plain) or m * n * k < 2 ** 24
 
 
-def test_f32_on_the_tensor_cores_is_exact_on_integers():
+def test_f32_on_the_tensor_cores_is_exact_on_integers(monkeypatch):
     """Integers below 2^24 are sums of three bf16 terms exactly, their products
     and sums below 2^24 are exact in f32: no tolerance."""
+    monkeypatch.setenv("VXB_F32_TENSOR", "1")
     rng = np.random.default_rng(77)
     a = rng.integers(-2000, 2000, (256, 256)).astype(np.float32)
     b = rng.integers(-3, 4, (256, 512)).astype(np.float32)
